@@ -82,7 +82,7 @@ struct fb_disk {
   cudaGraphExec_t exec[4];
   long long parts_run[4];
   uint64_t seq;                 /* begins so far: what the device reports with the CFL minimum */
-  int adv_pending;              /* the last advance's upload may not have been read yet */
+  int adv_pending;              /* PIN_ADVANCE may not have been read yet (host_scalars) */
   int feeldisk;                 /* some planet feels the disk */
   void *allocs[MAXALLOC];
   int nalloc;
@@ -1366,13 +1366,16 @@ int fb_disk_step_begin(fb_disk *D, double *cfl_min) {
 
 /* CflFluidsMin with the (global) CFL minimum, the DT clip (main.c:388-395)
  * and compute_potential's planetary update (potential.c:10-49); the step's
- * scalars into the pinned slot, whose last reader the wait of this step's
- * begin covered. */
+ * scalars into the pinned slot, once the copy that last read them there is
+ * known to be over: a begin has waited behind it, or the stream is waited for
+ * here (a step or an advance since the last begin). */
 static int host_scalars(fb_disk *D, double DT, double cfl_min, double *dt) {
   *dt = fb_psys_step(&D->ps, cfl_min, DT, &D->sc, D->feeldisk ? D->h_dtmin + 8 : NULL);
   if (*dt < 0.0) return fail(FB_ERR_NULL_DT, "null time step (CFL minimum %g)", cfl_min);
   D->sc.omegaframe = D->ps.omegaframe;
   D->sc.omegaframe0 = D->ps.omegaframe0;
+  if (D->adv_pending) CU(cudaStreamSynchronize(D->stream));
+  D->adv_pending = 1;
   memcpy((char *)D->h_dtmin + PIN_ADVANCE, &D->sc, sizeof(fb_scalars));
   return FB_OK;
 }
@@ -1383,8 +1386,6 @@ int fb_disk_step_advance(fb_disk *D, double DT, double cfl_min, double *dt_out) 
   double dt;
   if (!D) return fail(FB_ERR_ARG, "null disk");
   CU(cudaSetDevice(D->device));
-  if (D->adv_pending) CU(cudaStreamSynchronize(D->stream));   /* an advance without a begin since the last one */
-  D->adv_pending = 1;
   if ((rc = host_scalars(D, DT, cfl_min, &dt)) || (rc = run_part(D, PART_ADVANCE))) return rc;
   if (dt_out) *dt_out = dt;
   if (D->p.slab_ny_global > 0) CU(cudaStreamSynchronize(D->stream));   /* V_temp is read for the halos */

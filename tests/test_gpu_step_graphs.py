@@ -88,3 +88,28 @@ def test_changed_tiles_and_threads():
     for seed in (4, 5):
         for k in ("rho", "vx", "vy"):
             assert np.array_equal(out[seed][k], ref[seed][k])
+
+
+@pytest.mark.gpu
+def test_advances_without_a_begin():
+    """A whole step and then advances with the caller's own CFL minimum: the
+    same bits whether or not the stream is waited for between the calls."""
+    from fargo3d_b200 import Disk
+    got = []
+    for wait in (True, False):
+        d = Disk(_cfg(), "fp64")
+        d.load_initial_state()
+        dts = []
+        for n in range(8):
+            dts.append(d.step())
+            if wait:
+                d.state()
+            dts.append(d.step_advance(1e30, 0.5 * dts[-1]))
+            if wait:
+                d.state()
+            d.step_transport()
+        got.append((dts, d.state()))
+        d.close()
+    assert got[0][0] == got[1][0]
+    for k in ("rho", "vx", "vy"):
+        assert np.array_equal(got[0][1][k], got[1][1][k]), k

@@ -1,0 +1,87 @@
+"""The one-disk driver (fb_host.c) on a CUDA runtime of the host
+(fake_cuda.c), whose streams run as late as the real ones may: what a step
+queues reads what that step wrote."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture()
+def host(tmp_path):
+    if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
+        pytest.skip("no CUDA headers")
+    so = str(tmp_path / "libhost.so")   # a library of its own per test: its counters start at zero
+    subprocess.run(["gcc", "-O1", "-std=gnu99", "-fPIC", "-shared", "-ffp-contract=off", "-I" + os.path.join(CUDA, "include"),
+                    "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "fargo3d_b200", "csrc"),
+                    os.path.join(ROOT, "fargo3d_b200", "csrc", "fb_host.c"), os.path.join(ROOT, "tests", "fake_cuda.c"),
+                    "-o", so, "-lm", "-lpthread"], check=True)
+    L = C.CDLL(so)
+    L.fb_disk_stream.restype = C.c_void_p
+    L.fb_last_error.restype = C.c_char_p
+    L.fake_count.argtypes = [C.c_void_p]
+    return L
+
+
+class _Disk:
+    def __init__(self, L, **kw):
+        from fargo3d_b200 import _abi, config_fargo2d
+        self.L, self.h = L, C.c_void_p()
+        self.p = _abi.params_of(config_fargo2d(16, 8).replace(**kw))
+        self.check(L.fb_disk_create(C.byref(self.p), _abi.FB_FP64, 0, C.byref(self.h)))
+        self.stream = C.c_void_p(L.fb_disk_stream(self.h))
+
+    def check(self, rc):
+        assert rc == 0, self.L.fb_last_error()
+
+    def begin(self):
+        m = C.c_double()
+        self.check(self.L.fb_disk_step_begin(self.h, C.byref(m)))
+        return m.value
+
+    def advance(self, cfl):
+        dt = C.c_double()
+        self.check(self.L.fb_disk_step_advance(self.h, C.c_double(1e30), C.c_double(cfl), C.byref(dt)))
+        return dt.value
+
+    def transport(self):
+        self.check(self.L.fb_disk_step_transport(self.h))
+
+    def step(self):
+        dt = C.c_double()
+        self.check(self.L.fb_disk_step(self.h, C.c_double(1e30), C.byref(dt)))
+        return dt.value
+
+    def sync(self):
+        assert self.L.cudaStreamSynchronize(self.stream) == 0
+
+    def close(self):
+        self.check(self.L.fb_disk_destroy(self.h))
+
+
+def _found(L):
+    return list((C.c_double * 256).in_dll(L, "fake_dts"))[:C.c_int.in_dll(L, "fake_ndts").value]
+
+
+@pytest.mark.parametrize("before", [0, 5])   # as launches, as graphs
+def test_each_step_reads_its_own_scalars(host, before):
+    """A whole step, then advances with the caller's own CFL minimum and no
+    begin between: the scalars of a step in flight stay until it has read
+    them."""
+    d = _Disk(host)
+    want = []
+    for _ in range(before):
+        want.append(d.step())
+        want.append(d.advance(0.5 * d.begin()))
+        d.transport()
+    want.append(d.step())
+    for k in range(3):
+        want.append(d.advance(0.01 * (k + 1)))
+        d.transport()
+    d.sync()
+    assert _found(host) == want
+    d.close()
