@@ -1199,22 +1199,23 @@ static int ghosts_fused(const fb_disk *D, int adiabatic_vtemp) {
   return !D->d.is3d && D->d.ny >= 4 && !adiabatic_vtemp;
 }
 
-/* The launches of a step's parts, queued on the disk's stream.  Part 1:
+/* The launches of a step's parts, queued on st: the disk's stream (the only
+ * one mark() records on), or run_part's while it captures.  Part 1:
  * ComputeVmed(Vx) + cfl (main.c:366-388), and the disk's pull on the planets
  * that feel it (AdvanceSystemFromDisk's accelerations, planets.c:86-114),
  * from the state at the step's start, reported to the slot. */
-static int queue_begin(fb_disk *D) {
+static int queue_begin(fb_disk *D, cudaStream_t st) {
   int n;
   mark(D, "start");
-  LCH(LAUNCH(rowsum, &D->d, 0, D->stream));   /* with the slot's uploads (begin_upload) */
+  LCH(LAUNCH(rowsum, &D->d, 0, st));   /* with the slot's uploads (begin_upload) */
   mark(D, "rowsum");
   if (D->feeldisk) {
     for (n = 0; n < D->ps.np; n++)
       if (D->ps.feeldisk[n])
-        LCH(LAUNCH(disk_force, &D->d, D->d.pts + 4 * n, D->d_ring3, D->d_facc + 3 * n, D->stream));
+        LCH(LAUNCH(disk_force, &D->d, D->d.pts + 4 * n, D->d_ring3, D->d_facc + 3 * n, st));
     mark(D, "disk_force");
   }
-  LCH(LAUNCH(cfl, &D->d, D->stream));         /* with the report (cfl_report) */
+  LCH(LAUNCH(cfl, &D->d, st));         /* with the report (cfl_report) */
   mark(D, "cfl");
   return FB_OK;
 }
@@ -1222,26 +1223,26 @@ static int queue_begin(fb_disk *D) {
 /* Part 2: the step's scalars, then Sources (algogas.c:30-120) with SubStep3
  * and the ghost fill of V_temp on the mesh's own edges, the implicit drag
  * (main.c:412-414) and the dust diffusion (main.c:417-419). */
-static int queue_advance(fb_disk *D) {
+static int queue_advance(fb_disk *D, cudaStream_t st) {
   CU(cudaMemcpyAsync(D->d.scal_dev, (char *)D->h_dtmin + PIN_ADVANCE, sizeof(fb_scalars), cudaMemcpyHostToDevice,
-                     D->stream));
+                     st));
   mark(D, "host_scalars");
-  LCH(LAUNCH(sources, &D->d, D->stream));
+  LCH(LAUNCH(sources, &D->d, st));
   mark(D, "sources");
   if (D->d.adiabatic) {   /* SubStep3 (algogas.c:82-84), before the ghost fill */
-    LCH(LAUNCH(substep3, &D->d, D->stream));
+    LCH(LAUNCH(substep3, &D->d, st));
     mark(D, "substep3");
   }
   if (!ghosts_fused(D, D->d.adiabatic)) {
-    LCH(LAUNCH(bnd, &D->d, 1, D->stream));
+    LCH(LAUNCH(bnd, &D->d, 1, st));
     mark(D, "bnd_vtemp");
   }
   if (D->p.nfluids > 1) {
-    LCH(LAUNCH(collisions, &D->d, D->stream));
+    LCH(LAUNCH(collisions, &D->d, st));
     mark(D, "collisions");
   }
   if (D->d.dust_diffusion && D->p.nfluids > 1) {
-    LCH(LAUNCH(dust_diffusion, &D->d, D->stream));
+    LCH(LAUNCH(dust_diffusion, &D->d, st));
     mark(D, "dust_diffusion");
   }
   return FB_OK;
@@ -1249,30 +1250,30 @@ static int queue_advance(fb_disk *D) {
 
 /* Part 3: Transport (algogas.c:135-159), NewVelocity + StockholmBoundary and
  * the ghost fill on the mesh's own edges (main.c:427-431). */
-static int queue_transport(fb_disk *D) {
-  LCH(LAUNCH(rowsum, &D->d, 1, D->stream));
+static int queue_transport(fb_disk *D, cudaStream_t st) {
+  LCH(LAUNCH(rowsum, &D->d, 1, st));
   mark(D, "rowsum_vtemp");
-  LCH(LAUNCH(sweep_cols, &D->d, D->stream));
+  LCH(LAUNCH(sweep_cols, &D->d, st));
   mark(D, "sweep_cols");
-  LCH(LAUNCH(sweep_x, &D->d, D->stream));
+  LCH(LAUNCH(sweep_x, &D->d, st));
   mark(D, "sweep_x");
   if (D->d.is3d) {   /* 2D: with the azimuthal sweep */
-    LCH(LAUNCH(newvel, &D->d, D->stream));
+    LCH(LAUNCH(newvel, &D->d, st));
     mark(D, "newvel");
   }
   if (!ghosts_fused(D, 0)) {
-    LCH(LAUNCH(bnd, &D->d, 0, D->stream));
+    LCH(LAUNCH(bnd, &D->d, 0, st));
     mark(D, "bnd");
   }
   return FB_OK;
 }
 
 enum { PART_BEGIN, PART_ADVANCE, PART_TRANSPORT, PART_REST };   /* REST: advance + transport */
-static int queue_part(fb_disk *D, int part) {
+static int queue_part(fb_disk *D, int part, cudaStream_t st) {
   int rc = FB_OK;
-  if (part == PART_BEGIN) return queue_begin(D);
-  if (part != PART_TRANSPORT) rc = queue_advance(D);
-  if (!rc && part != PART_ADVANCE) rc = queue_transport(D);
+  if (part == PART_BEGIN) return queue_begin(D, st);
+  if (part != PART_TRANSPORT) rc = queue_advance(D, st);
+  if (!rc && part != PART_ADVANCE) rc = queue_transport(D, st);
   return rc;
 }
 
@@ -1285,15 +1286,23 @@ static int queue_part(fb_disk *D, int part) {
 static int run_part(fb_disk *D, int part) {
   if (D->prof || D->parts_run[part] < 4) {
     D->parts_run[part]++;
-    return queue_part(D, part);
+    return queue_part(D, part, D->stream);
   }
   if (!D->exec[part]) {
+    /* Captured on a stream of its own: the disk's is in its caller's hands
+       (fb_disk_stream) and a batch's members share one, so another thread may
+       queue work on it meanwhile, which is not part of this graph. */
     cudaGraph_t g = NULL;
+    cudaStream_t cap;
     cudaError_t e;
-    int rc;
-    CU(cudaStreamBeginCapture(D->stream, cudaStreamCaptureModeThreadLocal));
-    rc = queue_part(D, part);
-    e = cudaStreamEndCapture(D->stream, &g);
+    int rc = FB_OK;
+    CU(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+    e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      rc = queue_part(D, part, cap);
+      e = cudaStreamEndCapture(cap, &g);
+    }
+    cudaStreamDestroy(cap);
     if (rc || e != cudaSuccess) {
       if (g) cudaGraphDestroy(g);
       return rc ? rc : fail(FB_ERR_CUDA, "step graph capture: %s", cudaGetErrorString(e));

@@ -113,3 +113,40 @@ def test_advances_without_a_begin():
     assert got[0][0] == got[1][0]
     for k in ("rho", "vx", "vy"):
         assert np.array_equal(got[0][1][k], got[1][1][k]), k
+
+
+@pytest.mark.gpu
+def test_members_of_a_batch_on_their_own_threads():
+    """Members share the batch's stream: parts captured by one thread hold
+    nothing of what the other queues meanwhile."""
+    import ctypes as C
+    from fargo3d_b200 import Batch, Disk, _abi
+    ref = {}
+    for seed in (4, 5):
+        d = Disk(_cfg(seed=seed), "fp64")
+        d.load_initial_state()
+        ref[seed] = (d.run(40), d.state())
+        d.close()
+    b = Batch([_cfg(seed=4), _cfg(seed=5)], "fp64")
+    b.load_initial_states()
+    b.sync()
+    dts = {}
+
+    def work(i):
+        dt = C.c_double()
+        dts[4 + i] = []
+        for _ in range(40):
+            _abi.check(_abi.lib().fb_disk_step(b._members[i]._h, 1e30, C.byref(dt)))
+            dts[4 + i].append(dt.value)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for i, seed in enumerate((4, 5)):
+        assert dts[seed] == ref[seed][0]
+        st = b.state(i)
+        for k in ("rho", "vx", "vy"):
+            assert np.array_equal(st[k], ref[seed][1][k]), (seed, k)
+    b.close()

@@ -85,3 +85,24 @@ def test_each_step_reads_its_own_scalars(host, before):
     d.sync()
     assert _found(host) == want
     d.close()
+
+
+def test_work_queued_by_others_during_a_capture(host):
+    """A part is captured on a stream of its own: what another thread queues
+    on the disk's stream meanwhile (a batch's members share one) runs once."""
+    d = _Disk(host)
+    calls = []
+
+    @C.CFUNCTYPE(None)
+    def other():
+        calls.append(host.fake_count(d.stream))
+    C.c_void_p.in_dll(host, "fake_on_capture").value = C.cast(other, C.c_void_p).value
+    for _ in range(12):
+        d.advance(0.5 * d.begin())
+        d.transport()
+        d.step()
+    d.sync()
+    assert len(calls) >= 3   # begin, advance, transport
+    assert C.c_int.in_dll(host, "fake_counted").value == len(calls)
+    C.c_void_p.in_dll(host, "fake_on_capture").value = None
+    d.close()
