@@ -1223,9 +1223,8 @@ static int queue_begin(fb_disk *D, cudaStream_t st) {
 /* Part 2: the step's scalars, then Sources (algogas.c:30-120) with SubStep3
  * and the ghost fill of V_temp on the mesh's own edges, the implicit drag
  * (main.c:412-414) and the dust diffusion (main.c:417-419). */
-static int queue_advance(fb_disk *D, cudaStream_t st) {
-  CU(cudaMemcpyAsync(D->d.scal_dev, (char *)D->h_dtmin + PIN_ADVANCE, sizeof(fb_scalars), cudaMemcpyHostToDevice,
-                     st));
+static int queue_advance(fb_disk *D, cudaStream_t st, const void *sc) {
+  CU(cudaMemcpyAsync(D->d.scal_dev, sc, sizeof(fb_scalars), cudaMemcpyHostToDevice, st));
   mark(D, "host_scalars");
   LCH(LAUNCH(sources, &D->d, st));
   mark(D, "sources");
@@ -1269,12 +1268,18 @@ static int queue_transport(fb_disk *D, cudaStream_t st) {
 }
 
 enum { PART_BEGIN, PART_ADVANCE, PART_TRANSPORT, PART_REST };   /* REST: advance + transport */
-static int queue_part(fb_disk *D, int part, cudaStream_t st) {
+static int queue_part(fb_disk *D, int part, cudaStream_t st, const void *sc) {
   int rc = FB_OK;
   if (part == PART_BEGIN) return queue_begin(D, st);
-  if (part != PART_TRANSPORT) rc = queue_advance(D, st);
+  if (part != PART_TRANSPORT) rc = queue_advance(D, st, sc);
   if (!rc && part != PART_ADVANCE) rc = queue_transport(D, st);
   return rc;
+}
+
+/* whether the disk's stream is in a capture of its caller's */
+static int in_callers_capture(fb_disk *D) {
+  enum cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(D->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
 /* A part's launches never change from step to step (what changes travels in
@@ -1284,9 +1289,13 @@ static int queue_part(fb_disk *D, int part, cudaStream_t st) {
  * 384 x 128 one 60 -> 40).  The first ones go out as they are, so that a
  * disk's first steps do not wait for a capture. */
 static int run_part(fb_disk *D, int part) {
+  const void *sc = (char *)D->h_dtmin + PIN_ADVANCE;
+  /* a caller's graph takes the launches themselves, and its replays copy the
+     scalars the disk then has */
+  if (in_callers_capture(D)) return queue_part(D, part, D->stream, &D->sc);
   if (D->prof || D->parts_run[part] < 4) {
     D->parts_run[part]++;
-    return queue_part(D, part, D->stream);
+    return queue_part(D, part, D->stream, sc);
   }
   if (!D->exec[part]) {
     /* Captured on a stream of its own: the disk's is in its caller's hands
@@ -1299,7 +1308,7 @@ static int run_part(fb_disk *D, int part) {
     CU(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      rc = queue_part(D, part, cap);
+      rc = queue_part(D, part, cap, sc);
       e = cudaStreamEndCapture(cap, &g);
     }
     cudaStreamDestroy(cap);
@@ -1383,6 +1392,7 @@ static int host_scalars(fb_disk *D, double DT, double cfl_min, double *dt) {
   if (*dt < 0.0) return fail(FB_ERR_NULL_DT, "null time step (CFL minimum %g)", cfl_min);
   D->sc.omegaframe = D->ps.omegaframe;
   D->sc.omegaframe0 = D->ps.omegaframe0;
+  if (in_callers_capture(D)) return FB_OK;   /* run_part: the graph's copy reads D->sc */
   if (D->adv_pending) CU(cudaStreamSynchronize(D->stream));
   D->adv_pending = 1;
   memcpy((char *)D->h_dtmin + PIN_ADVANCE, &D->sc, sizeof(fb_scalars));

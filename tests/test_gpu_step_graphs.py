@@ -150,3 +150,30 @@ def test_members_of_a_batch_on_their_own_threads():
         for k in ("rho", "vx", "vy"):
             assert np.array_equal(st[k], ref[seed][1][k]), (seed, k)
     b.close()
+
+
+@pytest.mark.gpu
+def test_transport_inside_a_callers_capture():
+    import torch
+    from fargo3d_b200 import Disk
+    a, b = Disk(_cfg(), "fp64"), Disk(_cfg(), "fp64")
+    for d in (a, b):
+        d.load_initial_state()
+        for _ in range(6):   # the parts go out as graphs by now
+            d.step_advance(1e30, d.step_begin())
+            d.step_transport()
+        d.step_advance(1e30, d.step_begin())
+    a.step_transport()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(b.stream)):
+        g.capture_begin(capture_error_mode="thread_local")
+        b.step_transport()
+        g.capture_end()
+        g.replay()
+    for k in ("rho", "vx", "vy"):
+        assert np.array_equal(a.state()[k], b.state()[k]), k
+    assert a.step() == b.step()
+    del g
+    a.close()
+    b.close()

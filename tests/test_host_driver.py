@@ -106,3 +106,28 @@ def test_work_queued_by_others_during_a_capture(host):
     assert C.c_int.in_dll(host, "fake_counted").value == len(calls)
     C.c_void_p.in_dll(host, "fake_on_capture").value = None
     d.close()
+
+
+def test_parts_inside_a_callers_capture(host):
+    """A caller that captures the disk's stream gets the launches of advance
+    and transport in its graph, before and after they go out as graphs."""
+    d = _Disk(host)
+    for _ in range(7):
+        d.advance(d.begin())
+        d.transport()
+        d.step()
+        d.sync()
+        n = C.c_int.in_dll(host, "fake_ndts").value
+        g, e = C.c_void_p(), C.c_void_p()
+        assert host.cudaStreamBeginCapture(d.stream, 1) == 0
+        dt = d.advance(0.25)
+        d.transport()
+        assert host.cudaStreamEndCapture(d.stream, C.byref(g)) == 0
+        assert C.c_int.in_dll(host, "fake_ndts").value == n   # nothing ran yet
+        assert host.cudaGraphInstantiate(C.byref(e), g, C.c_ulonglong(0)) == 0
+        for _ in range(2):
+            assert host.cudaGraphLaunch(e, d.stream) == 0
+        d.sync()
+        assert _found(host)[n:] == [dt, dt]
+        assert host.cudaGraphDestroy(g) == 0 and host.cudaGraphExecDestroy(e) == 0
+    d.close()
