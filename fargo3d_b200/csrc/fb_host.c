@@ -15,6 +15,7 @@
 #include <pthread.h>
 #include <stdlib.h>
 #include <string.h>
+#include <time.h>
 
 #include <cuda_runtime_api.h>
 
@@ -1328,19 +1329,28 @@ static int run_part(fb_disk *D, int part) {
 }
 
 /* Wait until the device has reported this begin: the sequence number in the
- * slot, written after everything else.  Now and then the stream is asked
- * whether it still works, so that an error ends the wait. */
+ * slot, written after everything else.  The slot is watched for SPIN_NS, which
+ * covers the steps whose length a wait for the stream would add to noticeably
+ * (some us to a 2D disk's 20 to 100), and then the stream is waited for, by
+ * spinning, yielding or blocking as the process chose for the device: longer
+ * steps must not keep a core from other threads. */
+#define SPIN_NS 200000
+static long long now_ns(void) {
+  struct timespec t;
+  clock_gettime(CLOCK_MONOTONIC, &t);
+  return (long long)t.tv_sec * 1000000000 + t.tv_nsec;
+}
 static int wait_report(fb_disk *D) {
   const uint64_t *seq = (const uint64_t *)D->h_dtmin + 2;
+  long long end = now_ns() + SPIN_NS;
   unsigned spins = 0;
-  while (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq) {
-    if (++spins % 4096 == 0) {
-      cudaError_t e = cudaStreamQuery(D->stream);
-      if (e == cudaErrorNotReady) continue;
-      if (e != cudaSuccess) return fail(FB_ERR_CUDA, "step begin: %s", cudaGetErrorString(e));
+  cudaError_t e;
+  while (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq)
+    if (++spins % 64 == 0 && now_ns() > end) {
+      if ((e = cudaStreamSynchronize(D->stream)) != cudaSuccess)
+        return fail(FB_ERR_CUDA, "step begin: %s", cudaGetErrorString(e));
       if (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq) return fail(FB_ERR_CUDA, "step begin: no report");
     }
-  }
   return FB_OK;
 }
 

@@ -131,3 +131,15 @@ def test_parts_inside_a_callers_capture(host):
         assert _found(host)[n:] == [dt, dt]
         assert host.cudaGraphDestroy(g) == 0 and host.cudaGraphExecDestroy(e) == 0
     d.close()
+
+
+def test_a_long_begin_waits_as_the_process_chose(host):
+    """The begin watches for its report a while and then waits for the stream,
+    which yields or blocks as the device's flags say."""
+    C.c_int.in_dll(host, "fake_lazy_cfl").value = 1
+    d = _Disk(host)
+    for _ in range(6):
+        assert d.begin() == 0.125
+    assert C.c_int.in_dll(host, "fake_syncs").value >= 6
+    assert C.c_int.in_dll(host, "fake_queries").value == 0
+    d.close()
