@@ -13,6 +13,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <pthread.h>
+#include <sched.h>
 #include <stdlib.h>
 #include <string.h>
 #include <time.h>
@@ -1277,7 +1278,8 @@ static int queue_part(fb_disk *D, int part, cudaStream_t st, const void *sc) {
   return rc;
 }
 
-/* whether the disk's stream is in a capture of its caller's */
+/* whether the disk's stream is in a capture of its caller's (advance and
+ * transport only: a begin, and so a whole step, waits for the device) */
 static int in_callers_capture(fb_disk *D) {
   enum cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(D->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
@@ -1289,11 +1291,11 @@ static int in_callers_capture(fb_disk *D) {
  * launch (a step of a 64 x 32 disk among others' steps 55 -> 32 us, of a
  * 384 x 128 one 60 -> 40).  The first ones go out as they are, so that a
  * disk's first steps do not wait for a capture. */
-static int run_part(fb_disk *D, int part) {
+static int run_part(fb_disk *D, int part, int captured) {
   const void *sc = (char *)D->h_dtmin + PIN_ADVANCE;
   /* a caller's graph takes the launches themselves, and its replays copy the
      scalars the disk then has */
-  if (in_callers_capture(D)) return queue_part(D, part, D->stream, &D->sc);
+  if (captured) return queue_part(D, part, D->stream, &D->sc);
   if (D->prof || D->parts_run[part] < 4) {
     D->parts_run[part]++;
     return queue_part(D, part, D->stream, sc);
@@ -1329,11 +1331,14 @@ static int run_part(fb_disk *D, int part) {
 }
 
 /* Wait until the device has reported this begin: the sequence number in the
- * slot, written after everything else.  The slot is watched for SPIN_NS, which
- * covers the steps whose length a wait for the stream would add to noticeably
- * (some us to a 2D disk's 20 to 100), and then the stream is waited for, by
- * spinning, yielding or blocking as the process chose for the device: longer
- * steps must not keep a core from other threads. */
+ * slot, written after everything else.  The slot is watched without a break
+ * for SPIN_NS, which covers the steps that a few us more would be felt in (a 2D
+ * disk's take 20 to 100).  A longer wait must not keep a core from other
+ * threads: where the process asked the device's waits to block, it is the
+ * stream's wait, else the slot is watched with a yield each time (the
+ * stream's wait would return some 9 us later: a 512x256x48 FP32 step 1092 ->
+ * 1101 us), and now and then the stream is asked whether it still works, so
+ * that an error ends the wait. */
 #define SPIN_NS 200000
 static long long now_ns(void) {
   struct timespec t;
@@ -1342,15 +1347,27 @@ static long long now_ns(void) {
 }
 static int wait_report(fb_disk *D) {
   const uint64_t *seq = (const uint64_t *)D->h_dtmin + 2;
-  long long end = now_ns() + SPIN_NS;
-  unsigned spins = 0;
+  long long end = 0;
+  unsigned spins = 0, flags = 0;
   cudaError_t e;
-  while (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq)
-    if (++spins % 64 == 0 && now_ns() > end) {
-      if ((e = cudaStreamSynchronize(D->stream)) != cudaSuccess)
-        return fail(FB_ERR_CUDA, "step begin: %s", cudaGetErrorString(e));
-      if (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq) return fail(FB_ERR_CUDA, "step begin: no report");
+  while (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq) {
+    if (++spins % 256 != 0) continue;
+    if (!end) end = now_ns() + SPIN_NS;
+    if (now_ns() > end) break;
+  }
+  if (__atomic_load_n(seq, __ATOMIC_ACQUIRE) == D->seq) return FB_OK;
+  CU(cudaGetDeviceFlags(&flags));
+  for (spins = 0; __atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq; spins++) {
+    if ((flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync) {
+      e = cudaStreamSynchronize(D->stream);
+    } else {
+      sched_yield();
+      e = spins % 256 == 255 ? cudaStreamQuery(D->stream) : cudaErrorNotReady;
     }
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return fail(FB_ERR_CUDA, "step begin: %s", cudaGetErrorString(e));
+    if (__atomic_load_n(seq, __ATOMIC_ACQUIRE) != D->seq) return fail(FB_ERR_CUDA, "step begin: no report");
+  }
   return FB_OK;
 }
 
@@ -1382,7 +1399,7 @@ int fb_disk_step_begin(fb_disk *D, double *cfl_min) {
       pt[0] = x; pt[1] = y; pt[2] = z; pt[3] = sm;
     }
   D->nev = 0;
-  if ((rc = run_part(D, PART_BEGIN)) || (rc = wait_report(D))) return rc;
+  if ((rc = run_part(D, PART_BEGIN, 0)) || (rc = wait_report(D))) return rc;
   D->adv_pending = 0;
   if (((const uint64_t *)D->h_dtmin)[1] & 2)
     return fail(FB_ERR_NONFINITE, "a staged ring load of the azimuthal sweep did not complete in time");
@@ -1397,12 +1414,12 @@ int fb_disk_step_begin(fb_disk *D, double *cfl_min) {
  * scalars into the pinned slot, once the copy that last read them there is
  * known to be over: a begin has waited behind it, or the stream is waited for
  * here (a step or an advance since the last begin). */
-static int host_scalars(fb_disk *D, double DT, double cfl_min, double *dt) {
+static int host_scalars(fb_disk *D, double DT, double cfl_min, double *dt, int captured) {
   *dt = fb_psys_step(&D->ps, cfl_min, DT, &D->sc, D->feeldisk ? D->h_dtmin + 8 : NULL);
   if (*dt < 0.0) return fail(FB_ERR_NULL_DT, "null time step (CFL minimum %g)", cfl_min);
   D->sc.omegaframe = D->ps.omegaframe;
   D->sc.omegaframe0 = D->ps.omegaframe0;
-  if (in_callers_capture(D)) return FB_OK;   /* run_part: the graph's copy reads D->sc */
+  if (captured) return FB_OK;   /* run_part: the graph's copy reads D->sc */
   if (D->adv_pending) CU(cudaStreamSynchronize(D->stream));
   D->adv_pending = 1;
   memcpy((char *)D->h_dtmin + PIN_ADVANCE, &D->sc, sizeof(fb_scalars));
@@ -1411,11 +1428,12 @@ static int host_scalars(fb_disk *D, double DT, double cfl_min, double *dt) {
 
 /* Part 2 (queue_advance) */
 int fb_disk_step_advance(fb_disk *D, double DT, double cfl_min, double *dt_out) {
-  int rc;
+  int rc, captured;
   double dt;
   if (!D) return fail(FB_ERR_ARG, "null disk");
   CU(cudaSetDevice(D->device));
-  if ((rc = host_scalars(D, DT, cfl_min, &dt)) || (rc = run_part(D, PART_ADVANCE))) return rc;
+  captured = in_callers_capture(D);
+  if ((rc = host_scalars(D, DT, cfl_min, &dt, captured)) || (rc = run_part(D, PART_ADVANCE, captured))) return rc;
   if (dt_out) *dt_out = dt;
   if (D->p.slab_ny_global > 0) CU(cudaStreamSynchronize(D->stream));   /* V_temp is read for the halos */
   return FB_OK;
@@ -1436,7 +1454,7 @@ int fb_disk_step_transport(fb_disk *D) {
   int rc;
   if (!D) return fail(FB_ERR_ARG, "null disk");
   CU(cudaSetDevice(D->device));
-  if ((rc = run_part(D, PART_TRANSPORT)) || (rc = read_marks(D))) return rc;
+  if ((rc = run_part(D, PART_TRANSPORT, in_callers_capture(D))) || (rc = read_marks(D))) return rc;
   if (D->p.slab_ny_global > 0) CU(cudaStreamSynchronize(D->stream));   /* the state is read for the halos */
   return FB_OK;
 }
@@ -1444,7 +1462,7 @@ int fb_disk_step_transport(fb_disk *D) {
 int fb_disk_step(fb_disk *D, double DT, double *dt_out) {
   double cflmin = 0.0, dt;
   int rc = fb_disk_step_begin(D, &cflmin);
-  if (rc || (rc = host_scalars(D, DT, cflmin, &dt)) || (rc = run_part(D, PART_REST)) || (rc = read_marks(D))) return rc;
+  if (rc || (rc = host_scalars(D, DT, cflmin, &dt, 0)) || (rc = run_part(D, PART_REST, 0)) || (rc = read_marks(D))) return rc;
   if (dt_out) *dt_out = dt;
   if (D->p.slab_ny_global > 0) CU(cudaStreamSynchronize(D->stream));
   return FB_OK;

@@ -27,7 +27,7 @@ static void add(Ops *q, Op o) {
 
 /* what a test reads and sets */
 double fake_dts[256];          /* time steps the source launches found */
-int fake_ndts, fake_counted, fake_queries, fake_syncs, fake_lazy_cfl, fake_launches;
+int fake_ndts, fake_counted, fake_queries, fake_syncs, fake_yields, fake_lazy_cfl, fake_flags;
 void (*fake_on_capture)(void);
 
 static void run_op(const Op *o) {
@@ -57,7 +57,6 @@ static void drain(Stream *s) {
 static void queue(void *stream, Op o) {
   Stream *s = (Stream *)stream;
   int k, cfl = o.kind == CFL;
-  fake_launches++;
   if (s->capture) { add(s->capture, o); return; }
   add(&s->q, o);
   if (o.kind == GRAPH)
@@ -132,6 +131,8 @@ cudaError_t cudaMallocHost(void **p, size_t n) { *p = calloc(1, n); return cudaS
 cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { (void)d; return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDeviceFlags(unsigned *f) { *f = (unsigned)fake_flags; return cudaSuccess; }
+int fake_yield(void) { fake_yields++; return 0; }   /* fb_host.c is compiled with sched_yield as this */
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorStreamCaptureUnsupported ? "not permitted when stream is capturing" : "error"; }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = (cudaEvent_t)malloc(1); return cudaSuccess; }

@@ -16,8 +16,8 @@ def host(tmp_path):
     if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
         pytest.skip("no CUDA headers")
     so = str(tmp_path / "libhost.so")   # a library of its own per test: its counters start at zero
-    subprocess.run(["gcc", "-O1", "-std=gnu99", "-fPIC", "-shared", "-ffp-contract=off", "-I" + os.path.join(CUDA, "include"),
-                    "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "fargo3d_b200", "csrc"),
+    subprocess.run(["gcc", "-O1", "-std=gnu99", "-fPIC", "-shared", "-ffp-contract=off", "-Dsched_yield=fake_yield",
+                    "-I" + os.path.join(CUDA, "include"), "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "fargo3d_b200", "csrc"),
                     os.path.join(ROOT, "fargo3d_b200", "csrc", "fb_host.c"), os.path.join(ROOT, "tests", "fake_cuda.c"),
                     "-o", so, "-lm", "-lpthread"], check=True)
     L = C.CDLL(so)
@@ -133,13 +133,20 @@ def test_parts_inside_a_callers_capture(host):
     d.close()
 
 
-def test_a_long_begin_waits_as_the_process_chose(host):
-    """The begin watches for its report a while and then waits for the stream,
-    which yields or blocks as the device's flags say."""
+@pytest.mark.parametrize("flags", [0, 2, 4])   # automatic, yield, blocking
+def test_a_long_begin_leaves_the_core_to_others(host, flags):
+    """The begin watches for its report a while, then waits as the process
+    chose for the device: blocked in the stream's wait, or yielding."""
     C.c_int.in_dll(host, "fake_lazy_cfl").value = 1
+    C.c_int.in_dll(host, "fake_flags").value = flags
     d = _Disk(host)
+    now = [C.c_int.in_dll(host, "fake_" + n) for n in ("syncs", "queries", "yields")]
     for _ in range(6):
+        was = [n.value for n in now]
         assert d.begin() == 0.125
-    assert C.c_int.in_dll(host, "fake_syncs").value >= 6
-    assert C.c_int.in_dll(host, "fake_queries").value == 0
+        syncs, queries, yields = (n.value - w for n, w in zip(now, was))
+        if flags == 4:
+            assert (syncs, queries) == (1, 0)
+        else:
+            assert syncs == 0 and queries >= 1 and yields >= 100 * queries
     d.close()
