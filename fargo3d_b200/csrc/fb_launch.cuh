@@ -6,7 +6,28 @@
 namespace fb {
 
 // Each launch covers all the disk's fluids (one after the other they would
-// cost a launch each, with grids that leave most of the chip idle).
+// cost a launch each, with grids that leave most of the chip idle).  Where the
+// grid's third index counts layers or segments as well (per: those of one
+// fluid), it ends at 65535: launch(disk, fluids) is then called for as many
+// fluids at a time as fit.
+template <typename F>
+static int by_fluids(const fb_disk_dev *d, int per, F launch) {
+  const int nf = d->nfluids, most = per < 65535 ? 65535 / per : 1;
+  if (nf <= most) {
+    launch(*d, nf);
+    return (int)cudaGetLastError();
+  }
+  fb_disk_dev part = *d;
+  for (int f0 = 0; f0 < nf; f0 += most) {
+    part.nfluids = nf - f0 < most ? nf - f0 : most;
+    for (int f = 0; f < part.nfluids; f++) part.fl[f] = d->fl[f0 + f];
+    launch(part, part.nfluids);
+    const int e = (int)cudaGetLastError();
+    if (e) return e;
+  }
+  return 0;
+}
+
 template <typename T, typename S>
 static int launch_rowsum(const fb_disk_dev *d, int which, cudaStream_t st) {
   const int nring = d->sy * d->sz, nf = d->nfluids;
@@ -36,8 +57,11 @@ static int launch_sources(const fb_disk_dev *d, cudaStream_t st) {
     cudaGetDevice(&dev);
     if ((e = s3_allow<k_sources_sph<S>, S>(dev))) return e;
     const int layers = s3_layers((long long)s3_tiles(*d) * d->nz * nf, d->nz);
-    dim3 grid((nx + S3_TX - 1) / S3_TX, (ny + S3<S>::TY - 1) / S3<S>::TY, (d->nz + layers - 1) / layers * nf);
-    k_sources_sph<S><<<grid, S3<S>::T, sizeof(S3Shared<S>), st>>>(*d, layers);
+    const int segs = (d->nz + layers - 1) / layers;
+    return by_fluids(d, segs, [&](const fb_disk_dev &D, int n) {
+      dim3 grid((nx + S3_TX - 1) / S3_TX, (ny + S3<S>::TY - 1) / S3<S>::TY, segs * n);
+      k_sources_sph<S><<<grid, S3<S>::T, sizeof(S3Shared<S>), st>>>(D, layers);
+    });
   } else if constexpr (sizeof(S) == 4) {   // FP32 storage: FP32 arithmetic, column-marching warps
     const int rows = s32_rows((long long)nx * ny * nf);
     k_sources_cyl32<<<dim3((nx + S32_COLS - 1) / S32_COLS, (ny + rows - 1) / rows, nf), S32_WARPS * 32, 0, st>>>(*d, rows);
@@ -51,32 +75,33 @@ static int launch_sources(const fb_disk_dev *d, cudaStream_t st) {
 
 template <typename T, typename S>
 static int launch_bnd(const fb_disk_dev *d, int vtemp, cudaStream_t st) {
-  const int bx = 128, gx = (d->nx + bx - 1) / bx, nf = d->nfluids;
-  if (d->is3d) k_bnd_z<T, S><<<dim3(gx, d->sy, 6 * nf), bx, 0, st>>>(*d, vtemp);
-  k_bnd_y<T, S><<<dim3(gx, 6, d->sz * nf), bx, 0, st>>>(*d, vtemp);
-  return (int)cudaGetLastError();
+  const int bx = 128, gx = (d->nx + bx - 1) / bx;
+  if (d->is3d) k_bnd_z<T, S><<<dim3(gx, d->sy, 6 * d->nfluids), bx, 0, st>>>(*d, vtemp);
+  return by_fluids(d, d->sz, [&](const fb_disk_dev &D, int n) {
+    k_bnd_y<T, S><<<dim3(gx, 6, D.sz * n), bx, 0, st>>>(D, vtemp);
+  });
 }
 
 // radial sweep; in 3D the colatitude sweep (V_temp into set A) before it (set
 // A into set B)
 template <typename T, typename S>
 static int launch_sweep_cols(const fb_disk_dev *d, cudaStream_t st) {
-  const int ry = colm_rows(*d, 0);
-  auto grid = [&](int dir, int rows) {
-    dim3 g = colm_grid(*d, dir, rows);
-    g.z *= d->nfluids;
-    return g;
+  auto sweep = [&](int dir, auto kernel) {
+    const int rows = colm_rows(*d, dir);
+    const dim3 g = colm_grid(*d, dir, rows);
+    return by_fluids(d, (int)g.z, [&](const fb_disk_dev &D, int n) {
+      kernel<<<dim3(g.x, g.y, g.z * n), COL_T, 0, st>>>(D, rows);
+    });
   };
   if (d->is3d) {
-    const int rz = colm_rows(*d, 1);
-    k_sweep_colm<T, 1, true, false><<<grid(1, rz), COL_T, 0, st>>>(*d, rz);
-    k_sweep_colm<T, 0, true, false><<<grid(0, ry), COL_T, 0, st>>>(*d, ry);
-  } else if (d->adiabatic) {   // adiabatic disks transport their energy into e_a as a fifth quantity
-    if constexpr (sizeof(T) == 8) k_sweep_colm<T, 0, false, true><<<grid(0, ry), COL_T, 0, st>>>(*d, ry);
-  } else {
-    k_sweep_colm<T, 0, false, false><<<grid(0, ry), COL_T, 0, st>>>(*d, ry);
+    const int e = sweep(1, k_sweep_colm<T, 1, true, false>);
+    return e ? e : sweep(0, k_sweep_colm<T, 0, true, false>);
   }
-  return (int)cudaGetLastError();
+  if (d->adiabatic) {   // adiabatic disks transport their energy into e_a as a fifth quantity
+    if constexpr (sizeof(T) == 8) return sweep(0, k_sweep_colm<T, 0, false, true>);
+    return (int)cudaErrorInvalidValue;
+  }
+  return sweep(0, k_sweep_colm<T, 0, false, false>);
 }
 
 // The azimuthal sweep; in 2D with NewVelocity and Stockholm (fb_sweepx.cuh).
@@ -99,8 +124,9 @@ static int launch_sweep_x(const fb_disk_dev *d, cudaStream_t st) {
 template <typename T, typename S>
 static int launch_newvel(const fb_disk_dev *d, cudaStream_t st) {
   if (!d->is3d) return 0;
-  k_newvel<T, S><<<dim3((d->nx + 127) / 128, d->ny, d->nz * d->nfluids), 128, 0, st>>>(*d);
-  return (int)cudaGetLastError();
+  return by_fluids(d, d->nz, [&](const fb_disk_dev &D, int n) {
+    k_newvel<T, S><<<dim3((D.nx + 127) / 128, D.ny, D.nz * n), 128, 0, st>>>(D);
+  });
 }
 
 // implicit drag of all fluids (fluid count 2..FB_MAXFLUIDS)
