@@ -101,10 +101,20 @@ __device__ __forceinline__ double divk(double x, double y, double z) {
   return __fma_rn(__fma_rn(-y, q, x), z, q);
 }
 
-// n / d nearly correctly rounded (one residual step on the approximate
-// reciprocal): unbiased, as NewVelocity needs (b_newvel)
-__device__ __forceinline__ float div_res(float n, float d) {
-  const float z = __fdividef(1.0f, d), q = n * z;
+// RN(n / d): a Newton step on the approximate reciprocal gives RN(1 / d) (on
+// sm_100a for every mantissa, from exponent -110 to 110; test_gpu_div.py), and
+// with that the product and one residual step round as the division does
+// (Markstein), as long as quotient and remainder stay in the normal range.
+// NewVelocity divides by it: an error to one side would add up in a cell from
+// step to step.  64 disks' azimuthal sweep 208 us with the approximate
+// reciprocal alone (not always rounded so), 212 with the step, 215 with
+// __fdiv_rn; a 512x256x48 step 1102, 1102, 1117.
+__device__ __forceinline__ float recip_rn(float d) {
+  const float z = __fdividef(1.0f, d);
+  return fmaf(fmaf(-d, z, 1.0f), z, z);
+}
+__device__ __forceinline__ float div_rn(float n, float d) {
+  const float z = recip_rn(d), q = n * z;
   return fmaf(fmaf(-d, q, n), z, q);
 }
 
@@ -1044,14 +1054,14 @@ __device__ __forceinline__ void b_newvel(Dims m, Geo<T> g, const S *__restrict__
     // step after step); the azimuthal momenta are frame-relative, so the
     // OMEGAFRAME * R term is not subtracted.
     const T rc = m.sph ? ld(g.ymed + j) * ld(g.sin_zmed + k) : ld(g.ymed + j);
-    nvx = div_res((T)mmx[l] * sxi + (T)mpx[lxm] * sxim, (r * sxi + (T)rt[lxm] * sxim) * rc);
+    nvx = div_rn((T)mmx[l] * sxi + (T)mpx[lxm] * sxim, (r * sxi + (T)rt[lxm] * sxim) * rc);
     const T ivjm = ld(g.invvj + j - 1);
     const long long lym = l - m.pitch;
-    nvy = div_res((T)mmy[l] * ivjm + (T)mpy[lym] * ivj, r * ivjm + (T)rt[lym] * ivj);
+    nvy = div_rn((T)mmy[l] * ivjm + (T)mpy[lym] * ivj, r * ivjm + (T)rt[lym] * ivj);
     const T sykm = ld(g.syk + k - 1);
     const long long lzm = l - m.stride;
-    nvz = div_res((T)mmz[l] * syk + (T)mpz[lzm] * sykm, r * syk + (T)rt[lzm] * sykm);
-    if (m.sph) nvz = div_res(nvz, ld(g.ymed + j));
+    nvz = div_rn((T)mmz[l] * syk + (T)mpz[lzm] * sykm, r * syk + (T)rt[lzm] * sykm);
+    if (m.sph) nvz = div_rn(nvz, ld(g.ymed + j));
   } else {
     // the cells' volumes (times Sxi) are shared by the averages, and the
     // quotients by InvVj taken from its reciprocal

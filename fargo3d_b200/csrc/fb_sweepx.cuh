@@ -570,8 +570,8 @@ __device__ __forceinline__ void b_sweep_xs(const Dims &m, const Geo<T> &g, const
           // azimuthal momenta are relative to the frame and the background
 #pragma unroll
           for (int u = 0; u < C; u++) {
-            nvx[u] = div_res(outq[1][u] + (u ? outq[0][u - 1] : pxm), (out_r[u] + (u ? out_r[u - 1] : rxm)) * rc);
-            nvy[u] = div_res(outq[3][u] * ivjm + py_m[u] * ivj, out_r[u] * ivjm + r_m[u] * ivj);
+            nvx[u] = div_rn(outq[1][u] + (u ? outq[0][u - 1] : pxm), (out_r[u] + (u ? out_r[u - 1] : rxm)) * rc);
+            nvy[u] = div_rn(outq[3][u] * ivjm + py_m[u] * ivj, out_r[u] * ivjm + r_m[u] * ivj);
             nr[u] = out_r[u];
           }
         }
