@@ -432,9 +432,13 @@ static void drop_graphs(fb_disk *D) {
   }
 }
 
-/* Tile choices: azimuthal sweep cells per thread (1, 2, 4, 8, 16 dividing
- * Nx with at most 256 threads per ring; 0 restores the default) and column
- * sweep segment length (4, 8, 16; 0 restores 8). */
+/* Tile choices.  The column sweeps' segment length: 4, 8, 16, or 0, by the
+ * launch's work (col_rows).  The azimuthal sweep's cells per thread: 1, 2, 4,
+ * 8 or 16 that divide Nx into at most 256 threads and whose rings, as the
+ * kernel they belonged to staged them, fit a CTA's shared memory; 0 restores
+ * the default.  Its strips have one shape now: the value is checked, kept and
+ * reported as it always was, and the sweep takes the same rings (ring_fits),
+ * but nothing is tuned by it. */
 #define FB_SMEM_MAX (227 * 1024)
 
 static int default_cx(int nx) {
@@ -478,7 +482,7 @@ int fb_disk_set_wait_limit(fb_disk *D, long long polls) {
 int fb_disk_get_tiles(fb_disk *D, int *cx, int *ns) {
   if (!D) return fail(FB_ERR_ARG, "null disk");
   if (cx) *cx = D->d.tile_cx ? D->d.tile_cx : default_cx(D->d.nx);
-  if (ns) *ns = D->d.tile_ns ? D->d.tile_ns : (D->d.precision == FB_FP64 ? 4 : 8);
+  if (ns) *ns = D->d.tile_ns;
   return FB_OK;
 }
 

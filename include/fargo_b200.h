@@ -228,7 +228,8 @@ int fb_batch_poll(fb_batch *b, int *status, double *phys_time, long long *steps)
  * sweep_x_cells (1, 2, 4, 8 or 16, dividing Nx with at most 256 threads per
  * ring) is kept and has no effect any more, since the azimuthal sweep's strips
  * have a fixed shape; col_segment = cells per thread of the
- * radial/colatitude sweeps (4, 8 or 16); 0 = by the launch's work.  The
+ * radial/colatitude sweeps (4, 8 or 16); 0 = by the launch's work, and what
+ * fb_disk_get_tiles reports where none is set.  The
  * autotuner (fargo3d_b200/autotune.py) picks them per (Nx, Ny, Nz,
  * precision).  A batch member's choice takes effect at the next run. */
 int fb_disk_set_tiles(fb_disk *d, int sweep_x_cells, int col_segment);

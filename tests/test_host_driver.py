@@ -150,3 +150,21 @@ def test_a_long_begin_leaves_the_core_to_others(host, flags):
         else:
             assert syncs == 0 and queries >= 1 and yields >= 100 * queries
     d.close()
+
+
+def test_tiles_read_back(host):
+    """What get_tiles reports can be set again and changes nothing: 0 where the
+    launch's work decides the column segment."""
+    d = _Disk(host)
+    cx, ns = C.c_int(), C.c_int()
+
+    def get():
+        assert host.fb_disk_get_tiles(d.h, C.byref(cx), C.byref(ns)) == 0
+        return ns.value
+    assert get() == 0
+    for want in (4, 8, 16, 0):
+        d.check(host.fb_disk_set_tiles(d.h, 0, want))
+        assert get() == want
+        d.check(host.fb_disk_set_tiles(d.h, cx, ns))
+        assert get() == want
+    d.close()
