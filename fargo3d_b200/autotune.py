@@ -87,12 +87,19 @@ class TileTable:
         e = self.entries.get(shape_key(cfg, precision))
         return (e["sweep_x_cells"], e["col_segment"]) if e else None
 
+    def tiles(self, cfg, precision: str):
+        """The shape's tiles as fb_disk_set_tiles takes them: the azimuthal
+        width, which tunes nothing any more, 0 (the default) where it does not
+        tile the ring."""
+        t = self.get(cfg, precision)
+        return t and (t[0] if t[0] in cx_candidates(cfg.nx, precision, cfg.is3d) else 0, t[1])
+
     def apply(self, batch):
         """Set every member's tiles whose shape the table lists."""
         for i, c in enumerate(batch.cfgs):
-            t = self.get(c, batch.precision)
-            if t and t[0] in cx_candidates(c.nx, batch.precision, c.is3d):
-                batch.set_tiles(i, t[0], t[1])
+            t = self.tiles(c, batch.precision)
+            if t:
+                batch.set_tiles(i, *t)
 
     def save(self, path: str):
         os.makedirs(os.path.dirname(os.path.abspath(path)), exist_ok=True)

@@ -50,9 +50,9 @@ class Disk:
         _abi.check(L.fb_disk_create(C.byref(self._p), prec, device, C.byref(h)))
         self._h = h
         if tiles == "table":
-            from .autotune import TileTable, cx_candidates
-            t = TileTable.default().get(cfg, precision)
-            if t and t[0] in cx_candidates(cfg.nx, precision, cfg.is3d):
+            from .autotune import TileTable
+            t = TileTable.default().tiles(cfg, precision)
+            if t:
                 _abi.check(L.fb_disk_set_tiles(h, t[0], t[1]))
         self.shape = cfg.shape
 
