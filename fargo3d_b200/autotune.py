@@ -1,15 +1,14 @@
 """Tile autotuner: per disk shape and precision, the column sweeps' segment
-length that runs fastest (and the azimuthal sweep's tile, which the present
-kernel accepts but whose strips are as wide as its registers allow).
+length that runs fastest.  (The azimuthal sweep's cells per thread are kept in
+the table, and nothing depends on them: its strips are as wide as its
+registers allow.)
 
 The reference's GPU build picks one block shape per kernel by timing a sweep
 of shapes (scripts/blocks_function.py); here the choice is per disk shape,
 because a batch mixes shapes: a disk's tiles depend only on its own shape,
 never on the other members, so its arithmetic is the same alone and in any
-mix.  Each knob is timed in a batch of copies of the shape large enough to
-fill the GPU (one eager step per candidate, CUDA events per launch group,
-best of `reps`), the two knobs one after the other (the azimuthal sweep and
-the column sweeps are separate launches).
+mix.  Each candidate is timed in a batch of copies of the shape large enough
+to fill the GPU (one eager step, CUDA events per launch group, best of `reps`).
 
 Table: JSON {"<Nx>x<Ny>x<Nz>:<precision>": {"sweep_x_cells": C,
 "col_segment": NS, "ms": {...}}}.  `TileTable.default()` reads the table
@@ -108,8 +107,9 @@ class TileTable:
 
 
 def tune_shape(cfg, precision: str, device: int = 0, min_cells: float = 4e6, reps: int = 3, max_copies: int = 64):
-    """Time every candidate of both knobs for one shape; returns the table
-    entry.  The copies differ only in their noise seed."""
+    """Time the column segments for one shape; returns the table entry.  The
+    azimuthal sweep, which has one kernel whatever the width, is timed once and
+    keeps the library's width.  The copies differ only in their noise seed."""
     from .batch import Batch
     copies = int(min(max_copies, max(1, math.ceil(min_cells / cfg.active_cells))))
     cfgs = [cfg.replace(seed=cfg.seed + k) for k in range(copies)]
@@ -121,13 +121,11 @@ def tune_shape(cfg, precision: str, device: int = 0, min_cells: float = 4e6, rep
         t = min(b.profile_step()[group] for _ in range(reps))
         return t
 
-    ms_x = {}
-    for c in cx_candidates(cfg.nx, precision, cfg.is3d):
-        for i in range(copies):
-            b.set_tiles(i, c, 8)
-        b.profile_step()   # rebuild + warm
-        ms_x[c] = best("sweep_x")
-    cx = min(ms_x, key=ms_x.get)
+    cx = b.tiles(0)[0]
+    for i in range(copies):
+        b.set_tiles(i, cx, 8)
+    b.profile_step()   # rebuild + warm
+    ms_x = dict.fromkeys(cx_candidates(cfg.nx, precision, cfg.is3d), best("sweep_x"))
     ms_c = {}
     for ns in NS_CANDIDATES:
         for i in range(copies):

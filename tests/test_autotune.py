@@ -1,5 +1,6 @@
-"""The tile table on a stand-in batch: a tuned column segment is set whatever
-the table says of the azimuthal width."""
+"""The tile table and the tuner on a stand-in batch: a tuned column segment is
+set whatever the table says of the azimuthal width, and the tuner's width does
+not come from noise."""
 import pytest
 
 
@@ -39,3 +40,14 @@ def test_a_segment_is_set_with_any_width(width, want):
     t.apply(b)
     assert b.set == {0: (want, 8)}
     assert t.tiles(cfg, "fp64") == (want, 8) and t.tiles(b.cfgs[1], "fp64") is None
+
+
+def test_the_tuner_times_the_sweep_once(monkeypatch):
+    import fargo3d_b200.batch
+    from fargo3d_b200 import config_fargo2d
+    from fargo3d_b200.autotune import cx_candidates, tune_shape
+    monkeypatch.setattr(fargo3d_b200.batch, "Batch", _Batch)
+    e = tune_shape(config_fargo2d(256, 128), "fp32", min_cells=1, reps=2)
+    assert (e["sweep_x_cells"], e["col_segment"]) == (4, 8)   # the library's width, the fastest segment
+    assert set(e["ms"]["sweep_x"]) == {str(c) for c in cx_candidates(256, "fp32")}
+    assert len(set(e["ms"]["sweep_x"].values())) == 1
