@@ -64,12 +64,12 @@ METRIC = "cell-updates/s"
 ALG_WORDS = {"2d": 7, "3d": 9}
 # compulsory words per active cell of each launch group
 LAUNCH_WORDS = {
-    "2d": {"rowsum": 1, "cfl": 4, "sources": 6, "bnd_vtemp": 0, "rowsum_vtemp": 1,
-           "sweep_cols": 8, "sweep_x": 9, "bnd": 0, "scalars": 0},   # sweep_x: with the new velocities
+    "2d": {"rowsum": 1, "cfl": 4, "sources": 6, "rowsum_vtemp": 1,
+           "sweep_cols": 8, "sweep_x": 9, "scalars": 0},   # sweep_x: with the new velocities
     "3d": {"rowsum": 1, "cfl": 5, "sources": 8, "bnd_vtemp": 0, "rowsum_vtemp": 1,
            "sweep_cols": 26, "sweep_x": 15, "newvel": 11, "bnd": 0, "scalars": 0},
 }
-KERNELS_PER_GROUP = {"2d": {"sweep_cols": 1, "bnd": 1, "bnd_vtemp": 1, "dust_diffusion": 3},
+KERNELS_PER_GROUP = {"2d": {"dust_diffusion": 3},
                      "3d": {"sweep_cols": 2, "bnd": 2, "bnd_vtemp": 2}}
 
 

@@ -362,7 +362,7 @@ static int tiles(fb_batch *B, int st, std::vector<int4> &v, int chain = -1) {
         else g = dim3((nx + SRC2_TX - 1) / SRC2_TX, (ny + SRC2_TY - 1) / SRC2_TY);
         break;
       case ST_BND_Z: g = D.is3d ? dim3((nx + BND_BX - 1) / BND_BX, sy, 6) : dim3(0); break;
-      case ST_BND_Y: g = ghosts_fused(D.is3d, ny, 0) ? dim3(0) : dim3((nx + BND_BX - 1) / BND_BX, 6, sz); break;
+      case ST_BND_Y: g = D.is3d ? dim3((nx + BND_BX - 1) / BND_BX, 6, sz) : dim3(0); break;
       case ST_COLL: g = D.nfluids > 1 ? dim3((nx + 127) / 128, sy - 1, D.is3d ? sz - 1 : 1) : dim3(0); break;
       case ST_Z: case ST_Y: {
         if (st == ST_Z && !D.is3d) { g = dim3(0); break; }
@@ -462,9 +462,11 @@ static int launch_step(fb_batch *B, double DT, int chain) {
     kb_sources_cyl<<<grid(ST_SOURCES), SRC2_TX * SRC2_TY, 0, st>>>(ds, items[ST_SOURCES]);
   }
   pmark(st, "sources");
-  if (B->is3d) kb_bnd<T, S><<<grid(ST_BND_Z), BND_BX, 0, st>>>(ds, items[ST_BND_Z], 1, 1);
-  if (nitems[ST_BND_Y]) kb_bnd<T, S><<<grid(ST_BND_Y), BND_BX, 0, st>>>(ds, items[ST_BND_Y], 1, 0);
-  pmark(st, "bnd_vtemp");
+  if (B->is3d) {   // 2D: within the source stage
+    kb_bnd<T, S><<<grid(ST_BND_Z), BND_BX, 0, st>>>(ds, items[ST_BND_Z], 1, 1);
+    kb_bnd<T, S><<<grid(ST_BND_Y), BND_BX, 0, st>>>(ds, items[ST_BND_Y], 1, 0);
+    pmark(st, "bnd_vtemp");
+  }
   if (nf > 1 && nitems[ST_COLL]) {  // implicit drag between the fluids
     const int4 *it = items[ST_COLL];
     switch (nf) {
@@ -490,13 +492,13 @@ static int launch_step(fb_batch *B, double DT, int chain) {
   if (B->is3d) kb_sweep_xs<TX, 6, false><<<grid(ST_X), 32 * XS_WARPS, xs_smem<TX, XsC<TX>::C>(6), st>>>(ds, items[ST_X]);
   else kb_sweep_xs<TX, 4, true><<<grid(ST_X), 32 * XS_WARPS, xs_smem<TX, XsC<TX>::C>(4), st>>>(ds, items[ST_X]);
   pmark(st, "sweep_x");
-  if (B->is3d) {   // 2D: with the azimuthal sweep
+  if (B->is3d) {   // 2D: the new velocities and the state's ghosts are the azimuthal sweep's
     kb_newvel<TN, S><<<grid(ST_NEWVEL), NV_BX, 0, st>>>(ds, items[ST_NEWVEL]);
     pmark(st, "newvel");
     kb_bnd<T, S><<<grid(ST_BND_Z), BND_BX, 0, st>>>(ds, items[ST_BND_Z], 0, 1);
+    kb_bnd<T, S><<<grid(ST_BND_Y), BND_BX, 0, st>>>(ds, items[ST_BND_Y], 0, 0);
+    pmark(st, "bnd");
   }
-  if (nitems[ST_BND_Y]) kb_bnd<T, S><<<grid(ST_BND_Y), BND_BX, 0, st>>>(ds, items[ST_BND_Y], 0, 0);
-  pmark(st, "bnd");
   return (int)cudaGetLastError();
 }
 

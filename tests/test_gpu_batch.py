@@ -294,3 +294,17 @@ def test_batch_multifluid_drag_matches_oracle(precision):
                 l1 = np.sum(np.abs(st["rho"] - out[f]["rho"])) / np.sum(np.abs(out[f]["rho"]))
                 assert l1 <= 1e-5, (i, f, l1)
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_profiled_groups_are_those_that_launch(precision):
+    """A group is reported only where it launches something (the bench counts
+    launches by them): 2D ghosts are filled within other stages."""
+    from fargo3d_b200 import Batch, config_fargo2d, config_p3disof
+    stages = {"rowsum", "cfl", "scalars", "sources", "rowsum_vtemp", "sweep_cols", "sweep_x"}
+    for cfg, more in ((config_fargo2d(64, 16), set()), (config_p3disof(32, 8, 4), {"bnd_vtemp", "newvel", "bnd"})):
+        b = Batch([cfg, cfg], precision)
+        b.load_initial_states()
+        assert set(b.profile_step()) == stages | more
+        b.close()
