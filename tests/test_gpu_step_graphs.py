@@ -177,3 +177,26 @@ def test_transport_inside_a_callers_capture():
     del g
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,kind", [("fp32", "2d"), ("fp32", "3d"), ("fp64", "3d"), ("fp64", "adiabatic"),
+                                            ("fp64", "dust"), ("fp64", "diffusion"), ("fp32", "dust")])
+def test_captured_parts_are_the_launches(precision, kind):
+    """The same bits from launches (a profiled disk's steps) and from graphs,
+    of every kind of step."""
+    from fargo3d_b200 import Disk, _abi, config_adiabatic2d, config_multifluid, config_p3disof
+    cfg = {"2d": lambda: _cfg(True), "3d": lambda: config_p3disof(36, 12, 6, seed=2),
+           "adiabatic": lambda: config_adiabatic2d(48, 20, seed=2), "dust": lambda: config_multifluid(48, 20, nfluids=4),
+           "diffusion": lambda: config_multifluid(48, 20, nfluids=3, dust_diffusion=True)}[kind]().replace(noise=0.02)
+    got = []
+    for eager in (1, 0):
+        d = Disk(cfg, precision)
+        d.load_initial_state()
+        _abi.lib().fb_disk_profile(d._h, eager)
+        got.append((d.run(12), [d.state(f) for f in range(cfg.nfluids)]))
+        d.close()
+    assert got[0][0] == got[1][0]
+    for a, b in zip(got[0][1], got[1][1]):
+        for k in ("rho", "vx", "vy", "vz"):
+            assert np.array_equal(a[k], b[k]), k
