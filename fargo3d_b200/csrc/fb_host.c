@@ -1198,13 +1198,6 @@ int fb_disk_initialize(fb_disk *D) {
   return FB_OK;
 }
 
-/* 2D disks of at least four rows fill their ghosts within the source stage
- * (V_temp, where no SubStep3 comes between) and the azimuthal sweep (the
- * state): the rule of the kernels' ghosts_fused. */
-static int ghosts_fused(const fb_disk *D, int adiabatic_vtemp) {
-  return !D->d.is3d && D->d.ny >= 4 && !adiabatic_vtemp;
-}
-
 /* The launches of a step's parts, queued on st: the disk's stream (the only
  * one mark() records on), or run_part's while it captures.  Part 1:
  * ComputeVmed(Vx) + cfl (main.c:366-388), and the disk's pull on the planets
@@ -1238,7 +1231,7 @@ static int queue_advance(fb_disk *D, cudaStream_t st, const void *sc) {
     LCH(LAUNCH(substep3, &D->d, st));
     mark(D, "substep3");
   }
-  if (!ghosts_fused(D, D->d.adiabatic)) {
+  if (D->d.is3d || D->d.adiabatic) {   /* else within the source stage */
     LCH(LAUNCH(bnd, &D->d, 1, st));
     mark(D, "bnd_vtemp");
   }
@@ -1262,11 +1255,9 @@ static int queue_transport(fb_disk *D, cudaStream_t st) {
   mark(D, "sweep_cols");
   LCH(LAUNCH(sweep_x, &D->d, st));
   mark(D, "sweep_x");
-  if (D->d.is3d) {   /* 2D: with the azimuthal sweep */
+  if (D->d.is3d) {   /* 2D: the new velocities and the ghosts are the azimuthal sweep's */
     LCH(LAUNCH(newvel, &D->d, st));
     mark(D, "newvel");
-  }
-  if (!ghosts_fused(D, 0)) {
     LCH(LAUNCH(bnd, &D->d, 0, st));
     mark(D, "bnd");
   }

@@ -349,12 +349,6 @@ __device__ __forceinline__ float dmax3(float a, float b, float c) {
 }
 
 template <typename T>
-__device__ __forceinline__ T izsxmed(const Dims &m, const Geo<T> &g, int i, int j, int k) {
-  // Inv_zone_size_xmed
-  if (m.sph) return (ld(g.invdiffxmed + i) / ld(g.ymed + j) / ld(g.sin_zmed + k));
-  return (ld(g.invdiffxmed + i) / ld(g.ymed + j));
-}
-template <typename T>
 __device__ __forceinline__ T zsy(const Geo<T> &g, int j) { return (ld(g.ymin + j + 1) - ld(g.ymin + j)); }
 template <typename T>
 __device__ __forceinline__ T zsz(const Dims &m, const Geo<T> &g, int j, int k) {
@@ -526,63 +520,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 6) k_cfl(const __gri
 }
 
 // ---------------------------------------------------------------------------
-// Potential (potential.c:51-208), FP64, at one cell.
-__device__ __forceinline__ double potential_at(const Dims &m, const Geo<double> &gd,
-                                               const fb_scalars &sc, int i, int j, int k) {
-  double XC, YC, ZC, pot;
-  const double ym = ld(gd.ymed + j);
-  if (m.sph) {
-    XC = ym * ld(gd.cos_xmed + i) * ld(gd.sin_zmed + k);
-    YC = ym * ld(gd.sin_xmed + i) * ld(gd.sin_zmed + k);
-    ZC = ym * ld(gd.cos_zmed + k);
-    pot = -1.0 * 1.0 / ym;
-  } else {
-    XC = ym * ld(gd.cos_xmed + i);
-    YC = ym * ld(gd.sin_xmed + i);
-    ZC = ld(gd.zmed + k);
-    pot = -1.0 * 1.0 / sqrt(ym * ym + ZC * ZC);
-  }
-  for (int n = 0; n < sc.nplanets; n++) {
-    const double mp = sc.pmass[n] * 1.0;
-    const double xp = sc.px[n], yp = sc.py[n], zp = sc.pz[n];
-    const double dist = ((XC - xp) * (XC - xp) + (YC - yp) * (YC - yp) + (ZC - zp) * (ZC - zp));
-    if (sc.indirect_term) pot += 1.0 * mp * (XC * xp + YC * yp + ZC * zp) / sc.pdist3[n];
-    pot += -1.0 * mp / sqrt(dist + sc.psmooth2[n]);
-  }
-  return pot;
-}
-
-// The same potential for FP32-storage disks: the star's term from the per-row
-// table, the indirect term with the planets' m / d^3 precomputed (ind[n]),
-// the planets' terms with an FP64 reciprocal square root.
-__device__ __forceinline__ double potential_fast(const Dims &m, const Geo<double> &gd, const fb_scalars &sc,
-                                                 const double *ind, int i, int j, int k) {
-  double XC, YC, ZC;
-  const double ym = ld(gd.ymed + j);
-  if (m.sph) {
-    XC = ym * ld(gd.cos_xmed + i) * ld(gd.sin_zmed + k);
-    YC = ym * ld(gd.sin_xmed + i) * ld(gd.sin_zmed + k);
-    ZC = ym * ld(gd.cos_zmed + k);
-  } else {
-    XC = ym * ld(gd.cos_xmed + i);
-    YC = ym * ld(gd.sin_xmed + i);
-    ZC = ld(gd.zmed + k);
-  }
-  double pot = ld(gd.pot_star + j);
-  for (int n = 0; n < sc.nplanets; n++) {
-    const double xp = sc.px[n], yp = sc.py[n], zp = sc.pz[n];
-    const double dist = ((XC - xp) * (XC - xp) + (YC - yp) * (YC - yp) + (ZC - zp) * (ZC - zp));
-    if (sc.indirect_term) pot += ind[n] * (XC * xp + YC * yp + ZC * zp);
-    pot -= sc.pmass[n] * rsqrt(dist + sc.psmooth2[n]);
-  }
-  return pot;
-}
-
-}  // namespace fb
-
-namespace fb {
-
-// ---------------------------------------------------------------------------
 // Ghost cells from the setups' boundary templates (std/boundaries.txt with
 // setups/fargo/fargo.bound in 2D and setups/p3disof/p3disof.bound in 3D;
 // index rules of scripts/boundparser.py:360-398).  All libm factors of the
@@ -601,15 +538,14 @@ struct BndTab {
   __device__ double zw(int s, int kk) const { return t[18 + 6 * sz + 6 * sy + s * 3 + kk]; }
 };
 
-// 2D disks of at least four rows fill their radial ghosts from the kernels
-// that write the mirrored active rows (the source stage V_temp's, the
-// azimuthal sweep the state's) instead of in a launch of their own: the
-// ghosts of column i that row j's value determines, with b_bnd_y's formulas.
+// 2D disks fill their radial ghosts from the kernels that write the mirrored
+// active rows (the source stage V_temp's, but for adiabatic disks, whose
+// SubStep3 reads the outer edge face before it is filled; the azimuthal sweep
+// the state's) instead of in a launch of their own: the ghosts of column i that
+// row j's value determines, with b_bnd_y's formulas.  A disk has at least four
+// rows (fb_disk_create), of which one may mirror to both sides.
 // rho, e: null for V_temp / isothermal disks.  The caller stores vy = 0 on the
 // lower edge face (row Nghy) itself.
-__host__ __device__ inline bool ghosts_fused(int is3d, int ny, int adiabatic_vtemp) {
-  return !is3d && ny >= 4 && !adiabatic_vtemp;
-}
 template <typename S>
 __device__ __forceinline__ void ghosts_of_row(const Dims &m, const double *__restrict__ ymed, const double *__restrict__ tab,
                                               const double *__restrict__ vbg, double of, int i, int j, S *rho, S *vx,
@@ -788,7 +724,7 @@ __device__ __forceinline__ void b_sources_cyl(const Dims &m, const Geo<double> &
   ax += divk(-2.0 * dt * dxmed * (qx - qxm), dx_, idx_) * izx;
   ay += divk(-2.0 * (qy - qym), dy_, idy_) * dt;
   vxt[l] = ax;
-  if (ghosts_fused(0, m.ny, m.adiab)) {
+  if (!m.adiab) {
     vyt[l] = j == FB_NGH && m.bclo ? 0.0 : ay;
     if (edge_row(m, j)) ghosts_of_row<double>(m, g.ymed, tab, nullptr, of, i, j, nullptr, vxt, vyt, nullptr, r, ax, ay, 0.0);
   } else {
@@ -1417,26 +1353,16 @@ static __global__ void __launch_bounds__(256) k_mass_fold(const double *__restri
   }
 }
 
-// the chunk width a ring of nx cells uses with NT threads per CTA (0: none fits)
-__host__ __device__ inline int sweep_x_chunk(int nx, int nt) {
-  // the smallest of 4, 8, 16 that fits a ring into nt threads; odd rings 2, 1
-  const int cs[5] = {4, 8, 16, 2, 1};
-  for (int t = 0; t < 5; t++)
-    if (nx % cs[t] == 0 && nx / cs[t] <= nt) return cs[t];
-  return 0;
-}
-
-// Tile choices of a disk: the set value (fb_disk_set_tiles, usually from the
-// autotuner) or the default.
-inline int disk_cx(const fb_disk_dev &d) { return d.tile_cx ? d.tile_cx : sweep_x_chunk(d.nx, 256); }
-inline bool valid_cx(int nx, int c) { return (c == 1 || c == 2 || c == 4 || c == 8 || c == 16) && nx % c == 0 && nx / c <= 256; }
-inline bool valid_ns(int ns) { return ns == 4 || ns == 8 || ns == 16; }
-// the rings a step takes: an azimuthal tile of 1, 2, 4, 8 or 16 cells a thread
-// that divides them into at most 256 threads, and whose two buffers of every
-// quantity stay within an SM's shared memory (the rule of fb_disk_set_tiles)
+// The rings a step takes, a limit of the interface: an azimuthal tile of 1, 2,
+// 4, 8 or 16 cells a thread (fb_disk_set_tiles) that divides them into at most
+// 256 threads and whose rings, two buffers of every quantity, fit an SM's shared
+// memory.  The strips of the sweep would take any ring.
 inline bool ring_fits(const fb_disk_dev &d) {
-  const int c = disk_cx(d);
-  if (c == 0 || !valid_cx(d.nx, c)) return false;
+  int c = d.tile_cx;
+  const int cs[5] = {4, 8, 16, 2, 1};   // the default: the first that fits
+  for (int t = 0; t < 5 && !c; t++)
+    if (d.nx % cs[t] == 0 && d.nx / cs[t] <= 256) c = cs[t];
+  if (c == 0) return false;
   const size_t esz = d.precision == FB_FP64 ? 8 : 4, nq = d.is3d ? 6 : (d.adiabatic ? 5 : 4);
   return (size_t)(256 / (d.nx / c)) * (d.nx + 16 / esz) * (2 * (1 + nq) + 1) * esz <= 227 * 1024;
 }

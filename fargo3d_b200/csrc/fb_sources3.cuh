@@ -193,7 +193,8 @@ __device__ __forceinline__ void b_sources_sph(const Dims &m, const Geo<double> &
       s.bg[k % 3][tid] = bg_at(vbg, min(j0 - 1 + tid, m.sy - 1) + k * m.sy);
     }
   };
-  // potential.c:51-208 (potential_fast's products for FP32 storage)
+  // potential.c:51-208; FP32 storage: the indirect term with m / d^3 (ind), the
+  // planets' terms with an FP64 reciprocal root
   auto potential = [&](int k, int e, int li, int lj) {
     const double *L = s.lay[k % 3];
     const double ym = s.ym[lj], XC = ym * s.cx[li] * L[L3_SZM], YC = ym * s.sx[li] * L[L3_SZM], ZC = ym * L[L3_CZM];

@@ -214,12 +214,8 @@ __device__ __forceinline__ void b_sources_cyl32(const Dims m, const Geo<float> g
     if (writes) {
       const float u1 = fmaf(ax, dt, C0.u), v1 = fmaf(ay, dt, C0.vy);   // relative to the background, as the state
       *ou = u1;
-      if (ghosts_fused(0, m.ny, 0)) {
-        *ov = j == FB_NGH && m.bclo ? 0.0f : v1;
-        if (edge_row(m, j)) ghosts_of_row<float>(m, gd.ymed, tab, vbg, of, i, j, nullptr, vxt, vyt, nullptr, r, u1, v1, 0.0f);
-      } else {
-        *ov = v1;
-      }
+      *ov = j == FB_NGH && m.bclo ? 0.0f : v1;
+      if (edge_row(m, j)) ghosts_of_row<float>(m, gd.ymed, tab, vbg, of, i, j, nullptr, vxt, vyt, nullptr, r, u1, v1, 0.0f);
     }
     ou += m.pitch;
     ov += m.pitch;

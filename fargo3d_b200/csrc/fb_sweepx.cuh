@@ -590,12 +590,11 @@ __device__ __forceinline__ void b_sweep_xs(const Dims &m, const Geo<T> &g, const
           }
         }
         const long long l = l0 + oc;
-        const bool fused = ghosts_fused(0, m.ny, 0);
         put(A.s_rho + l, nr);
         put(A.s_vx + l, nvx);
         // the transported energy (stockholm.c leaves it alone)
         if (NQ == 5 && A.s_e) put(A.s_e + l, outq[NQ - 1]);
-        if (fused && edge_row(m, j)) {
+        if (edge_row(m, j)) {
 #pragma unroll
           for (int u = 0; u < C; u++)
             if (in_strip(u))
