@@ -14,8 +14,8 @@
 // Membership is by slots: a disk is added to a free slot, activated (state
 // uploaded, initialised), and removed when its caller is done with it.  The
 // device descriptor array and the per-disk planet systems are indexed by slot;
-// the work lists (the azimuthal sweep has one per chunk width) and the graph
-// depend on the active set and are rebuilt lazily at the next run.
+// the work lists and the graph depend on the active set and are rebuilt lazily
+// at the next run.
 #include "fb_batch.cuh"
 
 #include <stdio.h>
@@ -101,8 +101,7 @@ struct ListPack {
   }
 };
 
-// Work lists for the active set; drops
-// the captured graph.
+// Work lists for the active set; drops the captured graph.
 static int rebuild(fb_batch *B) {
   if (B->exec) { cudaGraphExecDestroy(B->exec); B->exec = nullptr; }
   B->graph_steps = 0;

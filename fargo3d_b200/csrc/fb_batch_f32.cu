@@ -1,7 +1,7 @@
-// FP32 batched stage kernels: FP32 storage; the source stage computes in FP64
-// (its viscous stresses in FP32), the transport stages and the CFL's per-cell
-// limits in the types below (approximate single-precision division and square
-// root where they compute in FP32); shift, ring means and the CFL minimum FP64.
+// FP32 batched stage kernels: FP32 storage.  2D sources, the transport stages,
+// NewVelocity and the CFL's per-cell limits compute in FP32 (approximate
+// division and root but for NewVelocity's division, div_rn); 3D sources, ghosts,
+// drag, shift, ring means, planets and the CFL minimum in FP64.
 #include "fb_batch.cuh"
 #ifndef FB_TC
 #define FB_TC float

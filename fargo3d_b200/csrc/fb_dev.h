@@ -22,7 +22,7 @@ typedef struct {
   /* frame-rotation radius tables (FP32 path): ymed^2, its row differences,
      sin^2(zmed) and its layer differences, differenced in double */
   const void *r2_j, *dr2_j, *s2_k, *ds2_k;
-  /* per-row reciprocals and the star's potential (FP32-storage sources):
+  /* per-row reciprocals and the star's potential (sources):
      1/Ymed, 1/Ymin, 1/(Ymed(j) - Ymed(j-1)), -G M / r at Ymed */
   const void *inv_ymed, *inv_ymin, *inv_dymed, *pot_star;
 } fb_geom_dev;
@@ -101,8 +101,8 @@ typedef struct {
   double *bnd_tab;        /* boundary factor tables (double) */
   int bnd_tab_n;
   double *ramps;          /* Stockholm ramps: [sy] radial, [sz] zmed, [sz] zmin */
-  int tile_cx;            /* azimuthal sweep cells per thread (0: default) */
-  int tile_ns;            /* column sweep segment length (0: default) */
+  int tile_cx;            /* azimuthal sweep cells per thread (0: default); tunes nothing (fb_disk_set_tiles) */
+  int tile_ns;            /* column sweep segment length (0: by the launch's work) */
   long long wait_limit;   /* polls of a bounded wait (0: default 2^22; < 0: none) */
   /* collision rates between the fluids, alpha[p + o * nfluids] (ColRate,
      colrate.c:10-23): alpha[0 + f n] = alpha[f + 0 n] = 1/St of dust fluid f */

@@ -104,12 +104,13 @@ __global__ void __launch_bounds__(256) k_cfl_static(fb_cfl_static_args a, const 
   }
 }
 
-// resets the running minimum to the MIN reduction's start value (1e20,
-// define.h:165) and the failure word before the rings are summed
+// the ring means of v_phi (compute_vmed.c:10-39), eight rings a warp
 __global__ void __launch_bounds__(32 * fb::RS_WARPS) k_rowsum_static(fb::Dims m, fb::Geo<double> gd, const double *v, double *out,
                                                        double xlen) {
   fb::b_rowsum<8>(m, gd, v, out, xlen, blockIdx.x, nullptr, nullptr);
 }
+// resets the running minimum to the MIN reduction's start value (1e20,
+// define.h:165) and the failure word before the rings are summed
 __global__ void k_reset_min(unsigned long long *dtmin) {
   dtmin[0] = 0x4415AF1D78B58C40ULL;
   dtmin[1] = 0ull;

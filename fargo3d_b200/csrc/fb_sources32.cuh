@@ -1,10 +1,12 @@
 // fb_sources32.cuh -- the source stage of FP32 2D cylindrical disks
 // (algogas.c:30-120: ComputePressureFieldIso, the planets' potential,
 // CorrectVtheta, SubStep1_x/y, visctensor_cyl + addviscosity_cyl, SubStep2_a/b)
-// in FP32 arithmetic, without shared memory or CTA barriers.
+// in FP32 arithmetic.  Cells pass through registers and shuffles; shared memory
+// holds what a row contributes and the planets, formed once per CTA before its
+// one barrier.
 //
 // Layout of the work: a warp owns 32 consecutive columns (azimuthal cells) of
-// a ring and marches down NS rows (radii), keeping the rows j-1, j, j+1 of its
+// a ring and marches over 2 to 16 rows (s32_rows), keeping j-1, j, j+1 of its
 // column in registers; the neighbours i-1 / i+1 come from the adjacent lanes
 // by shuffle.  Lanes 0 and 31 are halo lanes: they compute what their
 // neighbours need but write nothing, so a warp writes 30 columns.  Every
@@ -245,13 +247,13 @@ static __global__ void __launch_bounds__(S32_WARPS * 32, FB_S32_MINB) k_sources_
 }
 
 // ---------------------------------------------------------------------------
-// CFL time step of FP32 2D disks (cfl.c:135-258, cfl_b.c:14-39): the limits
-// of cfl_cell32 for a tile of 128 columns x CFL32_R rows, a lane per column
+// CFL time step of FP32 2D disks (cfl.c:135-258, cfl_b.c:14-39) whose rings
+// are no multiple of four cells: 128 columns x CFL32_R rows, a lane per column
 // marching over the rows with every load of the tile issued up front (the
 // kernel is a stream of four fields; it is bound by how many loads are in
 // flight), the x neighbour's vx by shuffle, the next row's vy reused.  The
 // tile's minimum (with the shear limits of its rows) is folded into the
-// disk's as in b_cfl; non-finite limits and non-positive densities set the
+// disk's by cfl_commit; non-finite limits and non-positive densities set the
 // disk's flag word.
 constexpr int CFL32_R = 8;
 

@@ -234,10 +234,10 @@ int fb_batch_poll(fb_batch *b, int *status, double *phys_time, long long *steps)
  * precision).  A batch member's choice takes effect at the next run. */
 int fb_disk_set_tiles(fb_disk *d, int sweep_x_cells, int col_segment);
 /* Failure detection of the azimuthal sweep's staged ring loads (no
- * counterpart in the reference, whose kernels never wait): a CTA polls the
+ * counterpart in the reference, whose kernels never wait): a warp polls the
  * copies' completion at most `polls` times (0: the default 2^22; negative:
- * not at all, the wait gives up at once).  A CTA that gives up waits,
- * boundedly again, for its copies to land, writes nothing and flags the
+ * not at all, the wait gives up at once).  A warp that gives up waits,
+ * boundedly again, for its copies to land, writes nothing more and flags the
  * disk; fb_disk_step reports FB_ERR_NONFINITE at the next step (the flag is
  * read with that step's CFL minimum), a batch freezes the member.  A batch
  * member takes the value its disk has when it is activated. */
