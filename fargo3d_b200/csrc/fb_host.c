@@ -139,6 +139,9 @@ static int dalloc(fb_disk *D, void **p, size_t bytes) {
  * flags, disk accelerations) and uploads, carved from 64 KiB pinned blocks and
  * recycled through a free list: creating a disk pins no memory of its own. */
 #define PIN_BLOCK (64 * 1024)
+_Static_assert(64 + 24 * FB_MAXPLANETS <= PIN_BEGIN && PIN_BEGIN + sizeof(fb_scalars) + 16 <= PIN_PTS &&
+                   PIN_PTS + 32 * FB_MAXPLANETS <= PIN_ADVANCE && PIN_ADVANCE + sizeof(fb_scalars) <= PIN_SLOT,
+               "the places of a slot");
 static pthread_mutex_t g_pin_mu = PTHREAD_MUTEX_INITIALIZER;
 static void *g_pin_free = NULL;             /* singly linked through the slots */
 static char *g_pin_block = NULL;
@@ -402,7 +405,7 @@ static int upload_tables(fb_disk *D) {
  * fields (exact) plus the per-row / per-layer tables (bounded). */
 int fb_params_bytes(const fb_params *p, int precision, size_t *out) {
   size_t esz, sy, sz, nc, rings, fields, b;
-  int is3d;
+  int is3d, n;
   if (!p || !out || p->nx < 1 || p->ny < 1 || p->nfluids < 1) return fail(FB_ERR_ARG, "invalid parameters");
   is3d = p->nz > 1;
   esz = precision == FB_FP64 ? sizeof(double) : sizeof(float);
@@ -417,6 +420,11 @@ int fb_params_bytes(const fb_params *p, int precision, size_t *out) {
   b += 2 * sizeof(double) * (6 * ((size_t)p->nx + 1) + 20 * (sy + 1) + 16 * (sz + 1));
   b += sizeof(double) * (18 + 6 * sz + 6 * sy + 6) + sizeof(double) * (sy + 2 * sz);
   b += 64 + sizeof(fb_scalars) + 64 * 16 + sizeof(double) * (2 * rings + 2);
+  for (n = 0; n < p->nplanets && n < FB_MAXPLANETS; n++)   /* the disk force's scratch (fb_disk_create) */
+    if (p->pl_feeldisk[n]) {
+      b += sizeof(double) * (3 * rings + 7 * FB_MAXPLANETS);
+      break;
+    }
   *out = b;
   return FB_OK;
 }

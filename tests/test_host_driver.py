@@ -168,3 +168,19 @@ def test_tiles_read_back(host):
         d.check(host.fb_disk_set_tiles(d.h, cx, ns))
         assert get() == want
     d.close()
+
+
+@pytest.mark.parametrize("feel", [False, True])
+@pytest.mark.parametrize("mesh", [(4, 4, 1), (4, 400, 1), (4, 4, 4), (4, 100, 100), (64, 12, 9)])
+def test_params_bytes_is_an_upper_bound(host, mesh, feel):
+    """What a disk requests stays within what fb_params_bytes says, with the
+    scratch of planets that feel the disk too."""
+    from fargo3d_b200 import Planet, _abi, config_fargo2d, config_p3disof
+    cfg = config_fargo2d(*mesh[:2]) if mesh[2] == 1 else config_p3disof(*mesh)
+    p = _abi.params_of(cfg.replace(planets=[Planet(1.0, 1e-3, True, True)]) if feel else cfg)
+    for prec in (_abi.FB_FP64, _abi.FB_FP32):
+        h, used, bound = C.c_void_p(), C.c_size_t(), C.c_size_t()
+        assert host.fb_disk_create(C.byref(p), prec, 0, C.byref(h)) == 0
+        assert host.fb_disk_bytes(h, C.byref(used)) == 0 and host.fb_params_bytes(C.byref(p), prec, C.byref(bound)) == 0
+        assert used.value <= bound.value
+        assert host.fb_disk_destroy(h) == 0
