@@ -1288,6 +1288,32 @@ static int in_callers_capture(fb_disk *D) {
   return cudaStreamIsCapturing(D->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
+/* The launches of a part as a graph, captured on a stream that only captures
+ * use: the disk's is in its caller's hands (fb_disk_stream) and a batch's
+ * members share one, so another thread may queue work on it meanwhile, which
+ * is not part of this graph.  One such stream per device, made on first use and
+ * kept for the life of the process (making and ending one takes some 100 us,
+ * more than a small disk's step), guarded by a lock; nothing ever runs on it. */
+static pthread_mutex_t g_cap_mu = PTHREAD_MUTEX_INITIALIZER;
+static cudaStream_t g_cap[FB_MAXDEV];
+static int capture_part(fb_disk *D, int part, const void *sc, cudaGraph_t *g) {
+  cudaError_t e = cudaSuccess;
+  int rc = FB_OK;
+  pthread_mutex_lock(&g_cap_mu);
+  if (!g_cap[D->device] && (e = cudaStreamCreateWithFlags(&g_cap[D->device], cudaStreamNonBlocking)) != cudaSuccess)
+    g_cap[D->device] = NULL;
+  if (e == cudaSuccess && (e = cudaStreamBeginCapture(g_cap[D->device], cudaStreamCaptureModeThreadLocal)) == cudaSuccess) {
+    rc = queue_part(D, part, g_cap[D->device], sc);
+    e = cudaStreamEndCapture(g_cap[D->device], g);
+  }
+  pthread_mutex_unlock(&g_cap_mu);
+  if (rc || e != cudaSuccess) {
+    if (*g) cudaGraphDestroy(*g);
+    return rc ? rc : fail(FB_ERR_CUDA, "step graph capture: %s", cudaGetErrorString(e));
+  }
+  return FB_OK;
+}
+
 /* A part's launches never change from step to step (what changes travels in
  * the pinned uploads), and each launch costs the host about 3.5 us, more than
  * most kernels of a 2D disk take: from the fifth time on a part is one graph
@@ -1299,29 +1325,15 @@ static int run_part(fb_disk *D, int part, int captured) {
   /* a caller's graph takes the launches themselves, and its replays copy the
      scalars the disk then has */
   if (captured) return queue_part(D, part, D->stream, &D->sc);
-  if (D->prof || D->parts_run[part] < 4) {
+  if (D->prof || D->parts_run[part] < 4 || D->device >= FB_MAXDEV) {
     D->parts_run[part]++;
     return queue_part(D, part, D->stream, sc);
   }
   if (!D->exec[part]) {
-    /* Captured on a stream of its own: the disk's is in its caller's hands
-       (fb_disk_stream) and a batch's members share one, so another thread may
-       queue work on it meanwhile, which is not part of this graph. */
     cudaGraph_t g = NULL;
-    cudaStream_t cap;
     cudaError_t e;
-    int rc = FB_OK;
-    CU(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-      rc = queue_part(D, part, cap, sc);
-      e = cudaStreamEndCapture(cap, &g);
-    }
-    cudaStreamDestroy(cap);
-    if (rc || e != cudaSuccess) {
-      if (g) cudaGraphDestroy(g);
-      return rc ? rc : fail(FB_ERR_CUDA, "step graph capture: %s", cudaGetErrorString(e));
-    }
+    int rc = capture_part(D, part, sc, &g);
+    if (rc) return rc;
     e = cudaGraphInstantiate(&D->exec[part], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
