@@ -24,8 +24,9 @@ enum { ST_ROWSUM, ST_CFL, ST_SOURCES, ST_BND_Z, ST_BND_Y, ST_COLL, ST_Z, ST_Y, S
 constexpr int CFL_R = 4, NV_R = 4;
 constexpr int BND_BX = 128, NV_BX = 128;
 
-// FP32 2D CFL (kb_cfl_cyl32): 6 CTAs of 128 threads per SM (80 registers);
-// the 64-disk step's CFL 0.090 -> 0.061 ms against the unconstrained 147
+// FP32 2D CFL of rings that are no multiple of four cells (kb_cfl_cyl32): 6
+// CTAs of 128 threads per SM (80 registers); on the 64-disk workload 0.090 ->
+// 0.061 ms against the unconstrained 147
 #ifndef FB_CFL32_MINB
 #define FB_CFL32_MINB 6
 #endif
@@ -274,8 +275,8 @@ static __global__ void kb_scalars(const fb_disk_dev *ds, fb_psys *ps, const int 
 using namespace fb;
 
 #define FB_MAX_CHAINS 8
-/* FP32 batches step as 4 concurrent chains (measured: 0.741 ms -> 0.684 ms for
-   the 64-disk workload); FP64 batches, whose stage kernels fill the GPU on
+/* FP32 batches step as 4 concurrent chains (64 disks: 0.460 -> 0.402 ms a step
+   against one); FP64 batches, whose stage kernels fill the GPU on
    their own, as one */
 #define FB_DEFAULT_CHAINS_F32 4
 #define FB_DEFAULT_CHAINS_F64 1
