@@ -15,8 +15,8 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 def host(tmp_path):
     if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
         pytest.skip("no CUDA headers")
-    so = str(tmp_path / "libhost.so")   # a library of its own per test: its counters start at zero
-    subprocess.run(["gcc", "-O1", "-std=gnu99", "-fPIC", "-shared", "-ffp-contract=off", "-Dsched_yield=fake_yield",
+    so = str(tmp_path / "libhost.so")   # a library of its own per test (its counters start at zero) that keeps to its own runtime
+    subprocess.run(["gcc", "-O1", "-std=gnu99", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-ffp-contract=off", "-Dsched_yield=fake_yield",
                     "-I" + os.path.join(CUDA, "include"), "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "fargo3d_b200", "csrc"),
                     os.path.join(ROOT, "fargo3d_b200", "csrc", "fb_host.c"), os.path.join(ROOT, "tests", "fake_cuda.c"),
                     "-o", so, "-lm", "-lpthread"], check=True)
