@@ -156,14 +156,14 @@ __device__ __forceinline__ void xs_ppa(const XsRing64<C> &R, const double *a, in
 }
 
 // ---- FP32: uniform zones; slopes in undivided differences, the PPA's edges
-// as deviations from the cell (no cancellation), the update factor folded
-// into the mass flux.  Algebraically the stages above.
+// as deviations from the cell (no cancellation), the update factor in the last
+// fused product of each pass.  Algebraically the stages above.
 template <int C>
 struct XsRing32 {
   float h0[C];        // 0.5 (1 - cr) upwind below, -0.5 (1 + cr) above
-  float f0[C], f1[C]; // v dt Surf / Vol; times the density face value once known
+  float f0[C];        // residual velocity
   bool up0[C];
-  float ks, up1;      // |v| dt / z of the rest velocity, its sign
+  float ks;           // |v| dt / z of the rest velocity
 };
 template <int C>
 __device__ __forceinline__ void xs_vl(const XsRing32<C> &R, const float *a, int lane, float *qs) {
@@ -470,17 +470,17 @@ __device__ __forceinline__ void b_sweep_xs(const Dims &m, const Geo<T> &g, const
       const float upd = rx.w;
       const bool up = rx.y > 0.0f;
       R.ks = fabsf(rx.y) * rx.z;
-      const float f1 = rx.y * upd;
+      const float f1 = rx.y;
 #pragma unroll
       for (int u = 0; u < C; u++) {
         const float v = vt[u] - rx.x, cr = v * rx.z;
         R.up0[u] = v > 0.0f;
         R.h0[u] = R.up0[u] ? 0.5f * (1.0f - cr) : -0.5f * (1.0f + cr);
-        R.f0[u] = v * upd;
+        R.f0[u] = v;
       }
-      // van Leer pass and rest pass of one quantity: x += flux differences;
-      // the flux of rho is f0 / f1 times its face value, of a momentum the
-      // density's flux times its own
+      // van Leer pass and rest pass of one quantity: x += upd times the flux
+      // differences; the flux of rho is f0 / f1 times its face value, of a
+      // momentum the density's flux times its own
       auto faces1 = [&](const float *a, float *fl) {   // PPA values at the C + 1 faces
         float gq[C];
         if (up) {
@@ -502,7 +502,7 @@ __device__ __forceinline__ void b_sweep_xs(const Dims &m, const Geo<T> &g, const
       fl[C] = from_right(m0[0], lane);
 #pragma unroll
       for (int u = 0; u < C; u++) {
-        rho1[u] = rho[u] + (m0[u] - (u < C - 1 ? m0[u + 1] : fl[C]));
+        rho1[u] = fmaf(m0[u] - (u < C - 1 ? m0[u + 1] : fl[C]), upd, rho[u]);
         ir0[u] = __fdividef(1.0f, rho[u]);
         ir1[u] = __fdividef(1.0f, rho1[u]);
       }
@@ -510,7 +510,7 @@ __device__ __forceinline__ void b_sweep_xs(const Dims &m, const Geo<T> &g, const
 #pragma unroll
       for (int u = 0; u <= C; u++) m1[u] *= f1;
 #pragma unroll
-      for (int u = 0; u < C; u++) out_r[u] = rho1[u] + (m1[u] - m1[u + 1]);
+      for (int u = 0; u < C; u++) out_r[u] = fmaf(m1[u] - m1[u + 1], upd, rho1[u]);
 #pragma unroll (NV ? NQ : 1)
       for (int q = 0; q < NQ; q++) {
         if (pre && q != 2) continue;
@@ -524,14 +524,14 @@ __device__ __forceinline__ void b_sweep_xs(const Dims &m, const Geo<T> &g, const
         fl[C] = from_right(fl[0], lane);
 #pragma unroll
         for (int u = 0; u < C; u++) {
-          x[u] = x[u] + (fl[u] - fl[u + 1]);
+          x[u] = fmaf(fl[u] - fl[u + 1], upd, x[u]);
           a[u] = x[u] * ir1[u];
         }
         faces1(a, fl);
 #pragma unroll
         for (int u = 0; u <= C; u++) fl[u] *= m1[u];
 #pragma unroll
-        for (int u = 0; u < C; u++) x[u] = x[u] + (fl[u] - fl[u + 1]);
+        for (int u = 0; u < C; u++) x[u] = fmaf(fl[u] - fl[u + 1], upd, x[u]);
         if constexpr (NV) {
 #pragma unroll
           for (int u = 0; u < C; u++) outq[q][u] = x[u];
