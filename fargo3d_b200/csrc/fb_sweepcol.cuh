@@ -58,7 +58,11 @@ __device__ __forceinline__ void b_sweep_colm(const Dims &m, const Geo<T> &g, con
     if (!m.sph) return ymed(c);
     return ymed(c) * (DIR == 0 ? st0 : ld(g.sin_zmed + c));
   };
+  // FP32 2D (the only sweep of four quantities): the row's zone size as it was
+  // differenced in double; a difference of two FP32 edges is off by up to
+  // 6e-8 Ymin / zone, the same in every step
   auto zone = [&](int c) -> T {
+    if (!F64 && NQ == 4) return ld(g.sxj + c);
     return DIR == 0 ? zsy(g, c) : zsz(m, g, t2, c);
   };
   // v Surf(c) (define.h:228-235, the macro's association); Syk = 1 in 2D

@@ -69,3 +69,54 @@ def test_fp64_batched_reference_follows_the_oracle(runs):
     for k in ("rho", "vx", "vy"):
         a, b = out["fp64"][i][k], ref[0][k]
         assert np.max(np.abs(a - b)) / np.max(np.abs(b)) <= 1e-8, (k,)
+
+
+@pytest.mark.gpu
+def test_roundings_of_ten_fp32_steps():
+    """The 64 disks' median relative L1 errors against FP64 after ten steps,
+    before the flow's own growth of differences shows.  The bounds are the
+    errors with one rounding per flux product and the update in a fused
+    product; one rounding a flux more reads 9.55e-8, 1.638e-9, 7.98e-5."""
+    from fargo3d_b200 import Batch, config_batched
+    cfgs = config_batched(64, 0)
+    st = {}
+    for prec in ("fp64", "fp32"):
+        b = Batch(cfgs, prec)
+        b.load_initial_states()
+        b.run(10)
+        b.sync()
+        st[prec] = [b.state(i) for i in range(64)]
+        b.close()
+    for k, bound in (("rho", 9.492e-8), ("vx", 1.6312e-9), ("vy", 7.889e-5)):
+        err = []
+        for w, g in zip(st["fp64"], st["fp32"]):
+            w, g = w[k][:, 3:-3], g[k][:, 3:-3]
+            err.append(np.abs(g - w).sum() / np.abs(w).sum())
+        assert np.median(err) <= bound, k
+
+
+@pytest.mark.gpu
+def test_fp32_ring_means_do_not_drift():
+    """What an FP32 disk's rings drift by in v_phi against FP64, with FP64's
+    own time steps: 1e-9 after 150 steps is the rounding of the state (6e-8 of
+    deviations of 1e-3 to 1e-2, a random walk over cells and steps).  Zone
+    sizes differenced in FP32 (6e-8 Ymin / zone, the same in every step) read
+    1.6e-9 to 1.9e-9."""
+    from fargo3d_b200 import Disk, config_fargo2d
+    drift = []
+    for s in range(4):
+        cfg = config_fargo2d((171, 160, 177, 172)[s], 90, seed=s).replace(noise=0.02)
+        d = Disk(cfg, "fp64")
+        d.load_initial_state()
+        dts = d.run(150)
+        w = d.state()["vx"][0, 3:-3]
+        d.close()
+        d = Disk(cfg, "fp32")
+        d.load_initial_state()
+        for dt in dts:
+            d.step_begin()
+            d.step_advance(1e30, dt)
+            d.step_transport()
+        drift.append(np.abs((d.state()["vx"][0, 3:-3] - w).mean(1)).mean())
+        d.close()
+    assert np.mean(drift) <= 1.25e-9, drift
