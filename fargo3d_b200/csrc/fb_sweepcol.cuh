@@ -44,6 +44,7 @@ __device__ __forceinline__ void b_sweep_colm(const Dims &m, const Geo<T> &g, con
                                              int c1, const fb_scalars *__restrict__ scp) {
   constexpr bool F64 = sizeof(T) == 8;
   constexpr int NA = NQ + (NE ? 1 : 0);
+  constexpr bool FLAT32 = !F64 && NQ == 4;   // the FP32 2D sweep
   const T dt = (T)scp->dt, of = (T)scp->omegaframe;
   const long long step = DIR == 0 ? (long long)m.pitch : m.stride;
   const long long base = DIR == 0 ? m.l(i, 0, t2) : m.l(i, t2, 0);
@@ -55,14 +56,13 @@ __device__ __forceinline__ void b_sweep_colm(const Dims &m, const Geo<T> &g, con
   // cylindrical radius and Ymed of cell c
   auto ymed = [&](int c) -> T { return DIR == 0 ? ld(g.ymed + c) : ym0; };
   auto radius = [&](int c) -> T {
-    if (!m.sph) return ymed(c);
+    if (FLAT32 || !m.sph) return ymed(c);
     return ymed(c) * (DIR == 0 ? st0 : ld(g.sin_zmed + c));
   };
-  // FP32 2D (the only sweep of four quantities): the row's zone size as it was
-  // differenced in double; a difference of two FP32 edges is off by up to
-  // 6e-8 Ymin / zone, the same in every step
+  // FP32 2D: the row's zone size as it was differenced in double; a difference
+  // of two FP32 edges is off by up to 6e-8 Ymin / zone, the same in every step
   auto zone = [&](int c) -> T {
-    if (!F64 && NQ == 4) return ld(g.sxj + c);
+    if (FLAT32) return ld(g.sxj + c);
     return DIR == 0 ? zsy(g, c) : zsz(m, g, t2, c);
   };
   // v Surf(c) (define.h:228-235, the macro's association); Syk = 1 in 2D
@@ -77,7 +77,7 @@ __device__ __forceinline__ void b_sweep_colm(const Dims &m, const Geo<T> &g, con
   // OMEGAFRAME (R^2(c) - R^2(c-1)) + (vbg R)(c) - (vbg R)(c-1)
   auto offs = [&](int c) -> T {
     T x;
-    if (!m.sph) x = ld(g.dr2_j + c);
+    if (FLAT32 || !m.sph) x = ld(g.dr2_j + c);
     else if (DIR == 0) x = ld(g.dr2_j + c) * ld(g.s2_k + t2);
     else x = ld(g.r2_j + t2) * ld(g.ds2_k + c);
     return of * x + (A.dl ? ld(A.dl + (DIR == 0 ? c + t2 * m.sy : t2 + c * m.sy)) : (T)0);
